@@ -176,9 +176,10 @@ int bounds_selftest(cudaStream_t s);
 size_t mlp_train_scratch_floats(int S);
 void mlp_loss_grad(const float* X, const float* y, int S, const float* w, float lo, float hi, float over,
                    float* scratch, float* grad, double* loss_out, cudaStream_t st);
-void mlp_adam_step(float* w, const float* grad, float* m, float* v, float lr, int step, cudaStream_t st);
-void mlp_predict(const float* X, int S, const float* w, float lo, float hi, float* scratch, float* pred,
-                 cudaStream_t st);
+// one full-batch epoch: the gradient and the Adam step number `step` on w
+void mlp_train_epoch(const float* X, const float* y, int S, float* w, float lo, float hi, float over, float* scratch,
+                     float* m, float* v, float lr, int step, cudaStream_t st);
+void mlp_predict(const float* X, int S, const float* w, float lo, float hi, float* pred, cudaStream_t st);
 // box: the domain box, or an ensemble's per-system boxes (nsys > 1, with
 // sys_off and the systems' level-1 cell ranges root_beg)
 // amag: each group's mean |a| of the previous evaluation (0 without one)

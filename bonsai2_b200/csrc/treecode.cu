@@ -1724,32 +1724,38 @@ int bonsai_get_group_theta(bonsai_handle hh, float* out) {
 }
 
 // standalone MLP training helpers (host arrays in and out)
+// one device allocation per call, carved into the arrays (cudaMalloc and
+// cudaFree of each by itself cost more than several epochs)
 struct MlpJob {
   float *X = nullptr, *y = nullptr, *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr, *scr = nullptr,
         *pred = nullptr;
   double* loss = nullptr;
+  char* slab = nullptr;
   cudaStream_t st = nullptr;
   ~MlpJob() {
-    dfree(&X); dfree(&y); dfree(&w); dfree(&g); dfree(&m); dfree(&v); dfree(&scr); dfree(&pred); dfree(&loss);
+    dfree(&slab);
     if (st) cudaStreamDestroy(st);
   }
   int init(int device, const float* hX, const float* hy, int S, const float* hw) {
     BONSAI_CUDA_TRY(cudaSetDevice(device));
     BONSAI_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    BONSAI_CUDA_TRY(dalloc(&X, (size_t)S * kMlpFeatures));
-    BONSAI_CUDA_TRY(dalloc(&y, (size_t)S));
-    BONSAI_CUDA_TRY(dalloc(&w, (size_t)kMlpWeights));
-    BONSAI_CUDA_TRY(dalloc(&g, (size_t)kMlpWeights));
-    BONSAI_CUDA_TRY(dalloc(&m, (size_t)kMlpWeights));
-    BONSAI_CUDA_TRY(dalloc(&v, (size_t)kMlpWeights));
-    BONSAI_CUDA_TRY(dalloc(&scr, mlp_train_scratch_floats(S)));
-    BONSAI_CUDA_TRY(dalloc(&pred, (size_t)S));
-    BONSAI_CUDA_TRY(dalloc(&loss, 1));
+    const size_t W = (size_t)kMlpWeights;
+    float** const arr[8] = {&X, &y, &w, &g, &m, &v, &scr, &pred};
+    const size_t len[8] = {(size_t)S * kMlpFeatures, (size_t)S, W, W, W, W, mlp_train_scratch_floats(S), (size_t)S};
+    size_t total = 256;  // the loss, then the arrays, each at a 256-byte boundary
+    for (int k = 0; k < 8; k++) total += (len[k] * sizeof(float) + 255) / 256 * 256;
+    BONSAI_CUDA_TRY(dalloc(&slab, total));
+    loss = reinterpret_cast<double*>(slab);
+    char* p = slab + 256;
+    for (int k = 0; k < 8; k++) {
+      *arr[k] = reinterpret_cast<float*>(p);
+      p += (len[k] * sizeof(float) + 255) / 256 * 256;
+    }
     BONSAI_CUDA_TRY(cudaMemcpyAsync(X, hX, (size_t)S * kMlpFeatures * 4, cudaMemcpyHostToDevice, st));
     if (hy) BONSAI_CUDA_TRY(cudaMemcpyAsync(y, hy, (size_t)S * 4, cudaMemcpyHostToDevice, st));
-    BONSAI_CUDA_TRY(cudaMemcpyAsync(w, hw, (size_t)kMlpWeights * 4, cudaMemcpyHostToDevice, st));
-    BONSAI_CUDA_TRY(cudaMemsetAsync(m, 0, (size_t)kMlpWeights * 4, st));
-    BONSAI_CUDA_TRY(cudaMemsetAsync(v, 0, (size_t)kMlpWeights * 4, st));
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(w, hw, W * 4, cudaMemcpyHostToDevice, st));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(m, 0, W * 4, st));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(v, 0, W * 4, st));
     return 0;
   }
 };
@@ -1775,10 +1781,7 @@ int bonsai_mlp_train(int device, const float* X, const float* y, int S, float* w
   MlpJob j;
   int rc = j.init(device, X, y, S, w);
   if (rc) return rc;
-  for (int e = 1; e <= epochs; e++) {
-    mlp_loss_grad(j.X, j.y, S, j.w, lo, hi, over, j.scr, j.g, nullptr, j.st);
-    mlp_adam_step(j.w, j.g, j.m, j.v, lr, e, j.st);
-  }
+  for (int e = 1; e <= epochs; e++) mlp_train_epoch(j.X, j.y, S, j.w, lo, hi, over, j.scr, j.m, j.v, lr, e, j.st);
   mlp_loss_grad(j.X, j.y, S, j.w, lo, hi, over, j.scr, j.g, j.loss, j.st);
   double l = 0;
   BONSAI_CUDA_TRY(cudaMemcpyAsync(w, j.w, (size_t)kMlpWeights * 4, cudaMemcpyDeviceToHost, j.st));
@@ -1793,8 +1796,7 @@ int bonsai_mlp_predict(int device, const float* X, int S, const float* w, float 
   MlpJob j;
   int rc = j.init(device, X, nullptr, S, w);
   if (rc) return rc;
-  BONSAI_CUDA_TRY(cudaMemsetAsync(j.pred, 0, (size_t)S * 4, j.st));
-  mlp_predict(j.X, S, j.w, lo, hi, j.scr, j.pred, j.st);
+  mlp_predict(j.X, S, j.w, lo, hi, j.pred, j.st);
   BONSAI_CUDA_TRY(cudaMemcpyAsync(theta, j.pred, (size_t)S * 4, cudaMemcpyDeviceToHost, j.st));
   BONSAI_CUDA_TRY(cudaStreamSynchronize(j.st));
   return last_cuda();

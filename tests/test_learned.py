@@ -56,6 +56,26 @@ def test_gpu_gradient_matches_oracle(lib):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("S", [1, 63, 64, 65, 148 * 64, 148 * 64 + 1, 30011])
+def test_gpu_gradient_sample_tiles(lib, S):
+    """Sizes around the 64-sample tiles and around one tile per block (148
+    blocks).  FP32 sums of at most S / 32 terms per thread: relative error
+    below S / 32 * 2^-24 of the sum of magnitudes, far under the bounds of the
+    test above."""
+    from oracle import mlp_oracle as M
+    from bonsai2_b200 import learned as Lr
+    X, y = _data(S, seed=S)
+    w = Lr.init_weights(2)
+    loss, g = Lr.loss_grad(X, y, w)
+    lo, go = M.loss_grad(X.astype(np.float64), y.astype(np.float64), w.astype(np.float64), LO, HI, OVER)
+    assert abs(loss - lo) <= 1e-5 * abs(lo)
+    assert np.allclose(g, go, rtol=1e-3, atol=1e-6 * np.abs(go).max())
+    th = Lr.predict(X, w)
+    to, _ = M.forward(X.astype(np.float64), w.astype(np.float64), LO, HI)
+    assert np.allclose(th, to, atol=2e-5)
+
+
+@pytest.mark.gpu
 def test_training_lowers_loss(lib):
     from bonsai2_b200 import learned as Lr
     rng = np.random.default_rng(3)
