@@ -44,17 +44,19 @@ int sort_timeout_selftest(cudaStream_t s);
 
 // tree.cu
 int tree_tiles(int n);
-void build_tree(const unsigned long long* sorted_keys, int n, int nleaf, int cell_cap, int leaf_cap, uint8_t* dlev,
-                uint16_t* chain, unsigned* hist, TreeInfo* info, uint4* cell_data, int* cell_parent, int* leaf_list,
-                int* mp_count, const int* sys_off, int nsys, int* root_beg, cudaStream_t s);
+size_t tree_hist_words(int n);
+// hist: tree_hist_words(n), zeroed once when allocated; cell_last: scratch, one int per cell
+void build_tree(const unsigned long long* sorted_keys, int n, int nleaf, int cell_cap, int leaf_cap, uint16_t* chain,
+                unsigned* hist, TreeInfo* info, uint4* cell_data, int* cell_parent, int* leaf_list, int* cell_last,
+                const int* sys_off, int nsys, int* root_beg, cudaStream_t s);
 
 // multipoles.cu
 // box: 6 floats per cell (float positions) or 6 doubles (jlo != nullptr:
 // double-single positions)
-void launch_multipoles(const int* leaf_list, const TreeInfo* info, const uint4* cell_data, const int* cell_parent,
-                       const float4* jpos, float inv_theta, MpRec* rec, void* box, float4* cell_open,
-                       float4* cell_stage, float4* cell_ls, int* mp_count, int cell_cap,
-                       const float4* jlo, float4* cell_lo, int nblocks, cudaStream_t s);
+void launch_multipoles(const int* leaf_list, const TreeInfo* info, const uint4* cell_data, const float4* jpos,
+                       float inv_theta, MpRec* rec, void* box, float4* cell_open, float4* cell_stage,
+                       float4* cell_ls, int cell_cap, const float4* jlo, float4* cell_lo, int nblocks,
+                       cudaStream_t s);
 __global__ void k_multipoles_ref_layout(const TreeInfo* __restrict__ info, const float4* __restrict__ cell_open,
                                         const MpRec* __restrict__ rec, float4* __restrict__ size,
                                         float4* __restrict__ mono, float4* __restrict__ quad0,

@@ -1,5 +1,5 @@
-// multipoles.cu -- monopole, quadrupole and opening size of every cell in one
-// launch, bottom up.
+// multipoles.cu -- monopole, quadrupole and opening size of every cell, bottom
+// up.
 //
 // The reference (computeCellMultipoles, computeMultipoles.cu:81-190) gives a
 // warp to every cell and rescans all of that cell's particles, O(N * depth)
@@ -7,8 +7,8 @@
 // reduced from its own particles (one thread per leaf, FP64, one pass: sums
 // about the leaf's first particle, shifted to the centre of mass), and every
 // node is combined from its
-// children with the parallel-axis theorem by the child that finishes last
-// (an arrival counter per cell; no thread waits on another).
+// children with the parallel-axis theorem, one launch per level from the
+// deepest.
 // Each particle is read once.  The quantities match the reference's definitions:
 //   M, COM; Q = second moment about the COM per unit mass (:148-158);
 //   particle bounding box -> l = max(2 max h, 1e-6), s = |cvec - COM|,
@@ -33,13 +33,6 @@ namespace bonsai {
 
 // leaf moments in one pass over the particles (1) or two (0: centre of mass,
 // then central moments)
-// parents level by level, one launch per level from the deepest (0: 6.55 ms
-// build phase at N = 2^24), or by the last-arriving child's climb with an
-// arrival counter per cell (1: 6.99 ms; fences and atomics serialise its
-// tail through the top levels); both bit-identical
-#ifndef BONSAI_MP_CLIMB
-#define BONSAI_MP_CLIMB 0
-#endif
 #ifndef BONSAI_MP_ONE_PASS
 #define BONSAI_MP_ONE_PASS 1
 #endif
@@ -121,64 +114,35 @@ __device__ __forceinline__ void store_cell(int c, const MpRec& r, const typename
   st[2] = make_float4(-(float)(3.0 * r.ixy), -(float)(3.0 * r.ixz), -(float)(3.0 * r.iyz), -t15);
 }
 
-// Arrival on a parent's counter: a fence publishes this child's record, a
-// relaxed atomic counts it, and only the last arriver fences again before it
-// reads its siblings' records (through L2).
-__device__ __forceinline__ bool arrive_last(int* p, int nch) {
-  __threadfence();
-  if (atomicAdd(p, 1) != nch - 1) return false;
-  __threadfence();
-  return true;
-}
-
-// A child's record fields.  CACHED (the level passes, whose children were
-// written by earlier launches): 16-byte vector loads through L1, so a record
-// costs 5 load instructions and its second read hits L1; otherwise (the
-// arrival-counter climb, whose siblings wrote them in this launch) 8-byte
-// loads from L2.
-template <bool CACHED>
+// A child's record fields (written by an earlier launch): 16-byte vector loads
+// through L1, so a record costs 5 load instructions and its second read hits
+// L1.
 __device__ __forceinline__ void load_mass_com(const MpRec* r, double& m, double& x, double& y, double& z) {
-  if (CACHED) {
-    const double2 a = __ldg(reinterpret_cast<const double2*>(r)), b = __ldg(reinterpret_cast<const double2*>(r) + 1);
-    m = a.x; x = a.y; y = b.x; z = b.y;
-  } else {
-    m = __ldcg(&r->m); x = __ldcg(&r->cx); y = __ldcg(&r->cy); z = __ldcg(&r->cz);
-  }
+  const double2 a = __ldg(reinterpret_cast<const double2*>(r)), b = __ldg(reinterpret_cast<const double2*>(r) + 1);
+  m = a.x; x = a.y; y = b.x; z = b.y;
 }
-template <bool CACHED>
 __device__ __forceinline__ MpRec load_rec(const MpRec* r) {
   MpRec o;
-  if (CACHED) {
-    const double2* q = reinterpret_cast<const double2*>(r);
-    const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3), e = __ldg(q + 4);
-    o.m = a.x; o.cx = a.y; o.cy = b.x; o.cz = b.y;
-    o.ixx = c.x; o.iyy = c.y; o.izz = d.x; o.ixy = d.y; o.ixz = e.x; o.iyz = e.y;
-  } else {
-    o.m = __ldcg(&r->m); o.cx = __ldcg(&r->cx); o.cy = __ldcg(&r->cy); o.cz = __ldcg(&r->cz);
-    o.ixx = __ldcg(&r->ixx); o.iyy = __ldcg(&r->iyy); o.izz = __ldcg(&r->izz);
-    o.ixy = __ldcg(&r->ixy); o.ixz = __ldcg(&r->ixz); o.iyz = __ldcg(&r->iyz);
-  }
+  const double2* q = reinterpret_cast<const double2*>(r);
+  const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3), e = __ldg(q + 4);
+  o.m = a.x; o.cx = a.y; o.cy = b.x; o.cz = b.y;
+  o.ixx = c.x; o.iyy = c.y; o.izz = d.x; o.ixy = d.y; o.ixz = e.x; o.iyz = e.y;
   return o;
 }
-template <bool CACHED, class B>
-__device__ __forceinline__ void load_box(const B* bk, B lo[3], B hi[3]) {
-  if (CACHED && sizeof(B) == 4) {
-    const float2* q = reinterpret_cast<const float2*>(bk);  // 24 B per cell: 8-byte aligned
-    const float2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-    lo[0] = (B)a.x; lo[1] = (B)a.y; lo[2] = (B)b.x; hi[0] = (B)b.y; hi[1] = (B)c.x; hi[2] = (B)c.y;
-  } else if (CACHED) {
-    const double2* q = reinterpret_cast<const double2*>(bk);  // 48 B per cell: 16-byte aligned
-    const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-    lo[0] = (B)a.x; lo[1] = (B)a.y; lo[2] = (B)b.x; hi[0] = (B)b.y; hi[1] = (B)c.x; hi[2] = (B)c.y;
-  } else {
-#pragma unroll
-    for (int a = 0; a < 3; a++) { lo[a] = __ldcg(bk + a); hi[a] = __ldcg(bk + 3 + a); }
-  }
+__device__ __forceinline__ void load_box(const float* bk, float lo[3], float hi[3]) {
+  const float2* q = reinterpret_cast<const float2*>(bk);  // 24 B per cell: 8-byte aligned
+  const float2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+  lo[0] = a.x; lo[1] = a.y; lo[2] = b.x; hi[0] = b.y; hi[1] = c.x; hi[2] = c.y;
+}
+__device__ __forceinline__ void load_box(const double* bk, double lo[3], double hi[3]) {
+  const double2* q = reinterpret_cast<const double2*>(bk);  // 48 B per cell: 16-byte aligned
+  const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+  lo[0] = a.x; lo[1] = a.y; lo[2] = b.x; hi[0] = b.y; hi[1] = c.x; hi[2] = c.y;
 }
 
 // A parent's moments from its nch contiguous children (parallel-axis
 // theorem, FP64), the children taken in index order.
-template <bool DS, bool CACHED>
+template <bool DS>
 __device__ void combine_children(int p, int first, int nch, float inv_theta, MpRec* __restrict__ rec,
                                  typename BoxOf<DS>::T* __restrict__ box, float4* __restrict__ cell_open,
                                  float4* __restrict__ cell_stage,
@@ -195,8 +159,8 @@ __device__ void combine_children(int p, int first, int nch, float inv_theta, MpR
 #pragma unroll
     for (int u = 0; u < kB; u++) {
       const int k = min(k0 + u, nch - 1);
-      load_mass_com<CACHED>(rec + first + k, mb[u], xb[u], yb[u], zb[u]);
-      load_box<CACHED>(box + 6 * (size_t)(first + k), lo[u], hi[u]);
+      load_mass_com(rec + first + k, mb[u], xb[u], yb[u], zb[u]);
+      load_box(box + 6 * (size_t)(first + k), lo[u], hi[u]);
     }
 #pragma unroll
     for (int u = 0; u < kB; u++) {
@@ -223,7 +187,7 @@ __device__ void combine_children(int p, int first, int nch, float inv_theta, MpR
     MpRec cb[kB2];
 #pragma unroll
     for (int u = 0; u < kB2; u++) {
-      cb[u] = load_rec<CACHED>(rec + first + min(k0 + u, nch - 1));
+      cb[u] = load_rec(rec + first + min(k0 + u, nch - 1));
     }
 #pragma unroll
     for (int u = 0; u < kB2; u++) {
@@ -243,28 +207,8 @@ __device__ void combine_children(int p, int first, int nch, float inv_theta, MpR
   store_cell<DS>(p, P, bmn, bmx, inv_theta, rec, box, cell_open, cell_stage, cell_ls, cell_lo);
 }
 
-// Combines parents bottom-up while this thread is the last child to arrive.
-template <bool DS>
-__device__ void climb(int c, [[maybe_unused]] int ncells, const uint4* __restrict__ cell_data,
-                      const int* __restrict__ cell_parent,
-                      float inv_theta, MpRec* __restrict__ rec, typename BoxOf<DS>::T* __restrict__ box,
-                      float4* __restrict__ cell_open, float4* __restrict__ cell_stage,
-                      float4* __restrict__ cell_ls, int* __restrict__ mp_count, float4* __restrict__ cell_lo) {
-  while (true) {
-    const int p = cell_parent[c];
-    if (p < 0) break;
-    if (!BONSAI_IN_RANGE(p, ncells, 0x303)) break;
-    const unsigned y = cell_data[p].y;
-    const int first = (int)(y & 0x1FFFFFFFu), nch = (int)(y >> 29) + 1;
-    if (!BONSAI_IN_RANGE(first + nch - 1, ncells, 0x304) || !BONSAI_IN_RANGE(c - first, nch, 0x305)) break;
-    if (!arrive_last(mp_count + p, nch)) break;
-    combine_children<DS, false>(p, first, nch, inv_theta, rec, box, cell_open, cell_stage, cell_ls, cell_lo);
-    c = p;
-  }
-}
-
 // The nodes of one level from their children, one thread per cell (leaves
-// were done by the leaf pass): the level-by-level form of the climb.
+// were done by the leaf pass).
 template <bool DS>
 __global__ void __launch_bounds__(256, BONSAI_MP_MINB) k_mp_level(int L, const TreeInfo* __restrict__ info,
                                                   const uint4* __restrict__ cell_data, float inv_theta,
@@ -279,21 +223,18 @@ __global__ void __launch_bounds__(256, BONSAI_MP_MINB) k_mp_level(int L, const T
     if (y == 0xFFFFFFFFu) continue;
     const int first = (int)(y & 0x1FFFFFFFu), nch = (int)(y >> 29) + 1;
     if (!BONSAI_IN_RANGE(first + nch - 1, ncells, 0x307)) continue;
-    combine_children<DS, true>(c, first, nch, inv_theta, rec, box, cell_open, cell_stage, cell_ls, cell_lo);
+    combine_children<DS>(c, first, nch, inv_theta, rec, box, cell_open, cell_stage, cell_ls, cell_lo);
   }
 }
 
-// One thread per leaf: the leaf's moments (one pass by default), then the
-// bottom-up climb.  (Half-warp-cooperative leaves
-// with shuffle reductions were measured 13x slower on the B200.)
-template <bool DS, bool CLIMB>
+// One thread per leaf: the leaf's moments (one pass by default).
+template <bool DS>
 __global__ void __launch_bounds__(256, BONSAI_MP_MINB) k_multipoles(const int* __restrict__ leaf_list, const TreeInfo* __restrict__ info,
                                                     const uint4* __restrict__ cell_data,
-                                                    const int* __restrict__ cell_parent,
                                                     const float4* __restrict__ jpos, float inv_theta,
                                                     MpRec* __restrict__ rec, typename BoxOf<DS>::T* __restrict__ box,
                                                     float4* __restrict__ cell_open, float4* __restrict__ cell_stage, float4* __restrict__ cell_ls,
-                                                    int* __restrict__ mp_count, int cell_cap,
+                                                    int cell_cap,
                                                     const float4* __restrict__ jlo, float4* __restrict__ cell_lo) {
   typedef typename BoxOf<DS>::T B;
   const int nleaves = info->nleaves;
@@ -396,44 +337,29 @@ __global__ void __launch_bounds__(256, BONSAI_MP_MINB) k_multipoles(const int* _
     r.m = m;
     r.ixx = q[0]; r.iyy = q[1]; r.izz = q[2]; r.ixy = q[3]; r.ixz = q[4]; r.iyz = q[5];
     store_cell<DS>(c, r, mn, mx, inv_theta, rec, box, cell_open, cell_stage, cell_ls, cell_lo);
-    if (CLIMB)
-      climb<DS>(c, ncells, cell_data, cell_parent, inv_theta, rec, box, cell_open, cell_stage, cell_ls, mp_count,
-                cell_lo);
   }
 }
 
-void launch_multipoles(const int* leaf_list, const TreeInfo* info, const uint4* cell_data, const int* cell_parent,
-                       const float4* jpos, float inv_theta, MpRec* rec, void* box, float4* cell_open,
-                       float4* cell_stage, float4* cell_ls, int* mp_count, int cell_cap,
-                       const float4* jlo, float4* cell_lo, int nblocks, cudaStream_t s) {
-#if BONSAI_MP_CLIMB
-  if (jlo)
-    k_multipoles<true, true><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, cell_parent, jpos, inv_theta, rec,
-                                                     static_cast<double*>(box), cell_open, cell_stage, cell_ls,
-                                                     mp_count, cell_cap, jlo, cell_lo);
-  else
-    k_multipoles<false, true><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, cell_parent, jpos, inv_theta, rec,
-                                                      static_cast<float*>(box), cell_open, cell_stage, cell_ls,
-                                                      mp_count, cell_cap, nullptr, nullptr);
-#else
+void launch_multipoles(const int* leaf_list, const TreeInfo* info, const uint4* cell_data, const float4* jpos,
+                       float inv_theta, MpRec* rec, void* box, float4* cell_open, float4* cell_stage,
+                       float4* cell_ls, int cell_cap, const float4* jlo, float4* cell_lo, int nblocks,
+                       cudaStream_t s) {
   // leaves, then the nodes level by level from the deepest (levels 20 .. 1)
-  const int lb = nblocks;
   if (jlo) {
-    k_multipoles<true, false><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, cell_parent, jpos, inv_theta, rec,
-                                                      static_cast<double*>(box), cell_open, cell_stage, cell_ls,
-                                                      mp_count, cell_cap, jlo, cell_lo);
+    k_multipoles<true><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, jpos, inv_theta, rec,
+                                               static_cast<double*>(box), cell_open, cell_stage, cell_ls, cell_cap,
+                                               jlo, cell_lo);
     for (int L = kMaxLevel - 1; L >= 1; L--)
-      k_mp_level<true><<<lb, 256, 0, s>>>(L, info, cell_data, inv_theta, rec, static_cast<double*>(box), cell_open,
-                                          cell_stage, cell_ls, cell_cap, cell_lo);
+      k_mp_level<true><<<nblocks, 256, 0, s>>>(L, info, cell_data, inv_theta, rec, static_cast<double*>(box),
+                                               cell_open, cell_stage, cell_ls, cell_cap, cell_lo);
   } else {
-    k_multipoles<false, false><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, cell_parent, jpos, inv_theta,
-                                                       rec, static_cast<float*>(box), cell_open, cell_stage,
-                                                       cell_ls, mp_count, cell_cap, nullptr, nullptr);
+    k_multipoles<false><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, jpos, inv_theta, rec,
+                                                static_cast<float*>(box), cell_open, cell_stage, cell_ls, cell_cap,
+                                                nullptr, nullptr);
     for (int L = kMaxLevel - 1; L >= 1; L--)
-      k_mp_level<false><<<lb, 256, 0, s>>>(L, info, cell_data, inv_theta, rec, static_cast<float*>(box), cell_open,
-                                           cell_stage, cell_ls, cell_cap, nullptr);
+      k_mp_level<false><<<nblocks, 256, 0, s>>>(L, info, cell_data, inv_theta, rec, static_cast<float*>(box),
+                                                cell_open, cell_stage, cell_ls, cell_cap, nullptr);
   }
-#endif
 }
 
 // Reference-layout view of the multipoles (debug/parity getter):

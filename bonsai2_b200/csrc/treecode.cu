@@ -68,13 +68,12 @@ struct Handle {
   unsigned long long* kalt2 = nullptr;
   int* valt2 = nullptr;
   unsigned* sort_counts2 = nullptr;
-  uint8_t* dlev = nullptr;
   uint16_t* chain = nullptr;
   unsigned* hist = nullptr;
   TreeInfo* info = nullptr;
   uint4* cell_data = nullptr;
   float4 *cell_open = nullptr, *cell_stage = nullptr;  // cell_stage: 3 per cell
-  int *cell_parent = nullptr, *leaf_list = nullptr, *mp_count = nullptr;
+  int *cell_parent = nullptr, *leaf_list = nullptr, *cell_last = nullptr;
   MpRec* rec = nullptr;
   double* cell_box = nullptr;  // 6 per cell: floats (float positions) or doubles (double-single)
   float4* cell_ls = nullptr;
@@ -247,7 +246,7 @@ struct Handle {
     dfree(&acc); dfree(&jpos); dfree(&tkey); dfree(&pkey); dfree(&kalt);
     dfree(&tperm); dfree(&pperm); dfree(&valt); dfree(&sort_counts); dfree(&bsum);
     dfree(&kalt2); dfree(&valt2); dfree(&sort_counts2);
-    dfree(&dlev); dfree(&chain); dfree(&hist); dfree(&groups); dfree(&group_inv); dfree(&group_tau); dfree(&group_amag);
+    dfree(&chain); dfree(&hist); dfree(&groups); dfree(&group_inv); dfree(&group_tau); dfree(&group_amag);
     dfree(&group_stats); dfree(&part_gid); dfree(&group_feat);
     dfree(&group_counts); dfree(&acc64); dfree(&acc64_tmp);
     release_cells();
@@ -255,7 +254,7 @@ struct Handle {
   }
   void release_cells() {
     dfree(&cell_data); dfree(&cell_open); dfree(&cell_stage);
-    dfree(&cell_parent); dfree(&leaf_list); dfree(&mp_count); dfree(&rec); dfree(&cell_ls);
+    dfree(&cell_parent); dfree(&leaf_list); dfree(&cell_last); dfree(&rec); dfree(&cell_ls);
     dfree(&cell_box);
     cap_cells = 0;
   }
@@ -290,7 +289,7 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&cell_stage, 3 * C));
     BONSAI_CUDA_TRY(dalloc(&cell_parent, C));
     BONSAI_CUDA_TRY(dalloc(&leaf_list, C));
-    BONSAI_CUDA_TRY(dalloc(&mp_count, C));
+    BONSAI_CUDA_TRY(dalloc(&cell_last, C));
     BONSAI_CUDA_TRY(dalloc(&rec, C));
     BONSAI_CUDA_TRY(dalloc(&cell_box, 6 * C));
     BONSAI_CUDA_TRY(dalloc(&cell_ls, C));
@@ -378,9 +377,9 @@ struct Handle {
     // scans: group counts per bin (8^7), and per position for ensembles (n)
     const int scan_m = std::max(std::max(256 * sort_tiles(nn), 1 << (3 * kMaxLevelSplit)), nn);
     BONSAI_CUDA_TRY(dalloc(&bsum, (size_t)scan_blocks(scan_m) + 1));
-    BONSAI_CUDA_TRY(dalloc(&dlev, N));
     BONSAI_CUDA_TRY(dalloc(&chain, N));
-    BONSAI_CUDA_TRY(dalloc(&hist, (size_t)2 * (kMaxLevel + 1) * tree_tiles(nn)));
+    BONSAI_CUDA_TRY(dalloc(&hist, tree_hist_words(nn)));
+    BONSAI_CUDA_TRY(cudaMemset(hist, 0, tree_hist_words(nn) * sizeof(unsigned)));
     BONSAI_CUDA_TRY(dalloc(&groups, N));
     // group-indexed arrays of the per-group angle: at most N/nCrit groups plus
     // one partial group per PH segment (groups.cu)
@@ -489,13 +488,12 @@ struct Handle {
     radix_sort_pairs(tkey, kalt, tperm, valt, nullptr, n, sort_counts, &info->status, 8, so(), nsys, st);
     k_gather_pos<<<nsm * 8, 256, 0, st>>>(tperm, n, pos[par], jpos);
     if (precision) k_gather_pos<<<nsm * 8, 256, 0, st>>>(tperm, n, plo[par], jlo);
-    build_tree(tkey, n, nleaf, cap_cells, cap_cells, dlev, chain, hist, info, cell_data, cell_parent, leaf_list,
-               mp_count, so(), nsys, root_beg, st);
+    build_tree(tkey, n, nleaf, cap_cells, cap_cells, chain, hist, info, cell_data, cell_parent, leaf_list, cell_last,
+               so(), nsys, root_beg, st);
   }
   void enq_multipoles() {
-    launch_multipoles(leaf_list, info, cell_data, cell_parent, jpos, 1.0f / prm.theta, rec, cell_box, cell_open,
-                      cell_stage, cell_ls, mp_count, cap_cells, precision ? jlo : nullptr,
-                      precision ? cell_lo : nullptr, nsm * 8, st);
+    launch_multipoles(leaf_list, info, cell_data, jpos, 1.0f / prm.theta, rec, cell_box, cell_open, cell_stage,
+                      cell_ls, cap_cells, precision ? jlo : nullptr, precision ? cell_lo : nullptr, nsm * 8, st);
   }
   void enq_groups(int ls, int ncrit) { enq_groups_on(ls, ncrit, st, kalt, valt, sort_counts); }
   void enq_groups_on(int ls, int ncrit, cudaStream_t s, unsigned long long* ka, int* va, unsigned* work) {
