@@ -53,10 +53,12 @@ void build_tree(const unsigned long long* sorted_keys, int n, int nleaf, int cel
 // multipoles.cu
 // box: 6 floats per cell (float positions) or 6 doubles (jlo != nullptr:
 // double-single positions)
-void launch_multipoles(const int* leaf_list, const TreeInfo* info, const uint4* cell_data, const float4* jpos,
+// barrier: one word of scratch; level_blocks: multipole_level_blocks of the device
+int multipole_level_blocks(int nsm);
+void launch_multipoles(const int* leaf_list, TreeInfo* info, const uint4* cell_data, const float4* jpos, int n,
                        float inv_theta, MpRec* rec, void* box, float4* cell_open, float4* cell_stage,
                        float4* cell_ls, int cell_cap, const float4* jlo, float4* cell_lo, int nblocks,
-                       cudaStream_t s);
+                       unsigned* barrier, int level_blocks, cudaStream_t s);
 __global__ void k_multipoles_ref_layout(const TreeInfo* __restrict__ info, const float4* __restrict__ cell_open,
                                         const MpRec* __restrict__ rec, float4* __restrict__ size,
                                         float4* __restrict__ mono, float4* __restrict__ quad0,

@@ -7,8 +7,7 @@
 // reduced from its own particles (one thread per leaf, FP64, one pass: sums
 // about the leaf's first particle, shifted to the centre of mass), and every
 // node is combined from its
-// children with the parallel-axis theorem, one launch per level from the
-// deepest.
+// children with the parallel-axis theorem, level by level from the deepest.
 // Each particle is read once.  The quantities match the reference's definitions:
 //   M, COM; Q = second moment about the COM per unit mass (:148-158);
 //   particle bounding box -> l = max(2 max h, 1e-6), s = |cvec - COM|,
@@ -46,37 +45,33 @@ struct BoxOf<true> {
   typedef double T;
 };
 
-// minimum blocks per SM of the leaf and level passes (1: no bound; 5 or 6
-// blocks spill the FP64 sums and were slower: build phase 4.59 / 4.84 ms
-// against 4.50 at N = 2^24)
-#ifndef BONSAI_MP_MINB
-#define BONSAI_MP_MINB 1
-#endif
 #ifndef BONSAI_MP_BATCH
 #define BONSAI_MP_BATCH 4
 #endif
 constexpr int kMpBatch = BONSAI_MP_BATCH;  // leaf particles loaded ahead of their sums
 
+// the walk's records of a cell
+struct CellOut {
+  float4 open, ls, stage[3], lo;
+};
 template <bool DS>
-__device__ __forceinline__ void store_cell(int c, const MpRec& r, const typename BoxOf<DS>::T* bmin,
-                                           const typename BoxOf<DS>::T* bmax, float inv_theta, MpRec* __restrict__ rec,
-                                           typename BoxOf<DS>::T* __restrict__ box, float4* __restrict__ cell_open,
-                                           float4* __restrict__ cell_stage,
-                                           float4* __restrict__ cell_ls, float4* __restrict__ cell_lo) {
-  rec[c] = r;
-  for (int k = 0; k < 3; k++) { box[6 * (size_t)c + k] = bmin[k]; box[6 * (size_t)c + 3 + k] = bmax[k]; }
+__device__ __forceinline__ CellOut cell_out(const MpRec& r, const typename BoxOf<DS>::T* bmin,
+                                            const typename BoxOf<DS>::T* bmax, float inv_theta) {
+  CellOut q;
   const float cx = (float)r.cx, cy = (float)r.cy, cz = (float)r.cz;
+  const double tr = r.ixx + r.iyy + r.izz;
+  const float t15 = (float)(1.5 * tr);
   float s, l;
   if (DS) {
     // w: the staged record's -0.5 tr I (cell_stage[3c].w), so that the
     // double-single walk, which loads cell_lo for every visited cell, stages
     // an accepted cell without another load
-    const float t15d = (float)(1.5 * (r.ixx + r.iyy + r.izz));
-    cell_lo[c] = make_float4((float)(r.cx - (double)cx), (float)(r.cy - (double)cy), (float)(r.cz - (double)cz),
-                             __fmul_rn(t15d, -1.0f / 3.0f));
+    q.lo = make_float4((float)(r.cx - (double)cx), (float)(r.cy - (double)cy), (float)(r.cz - (double)cz),
+                       __fmul_rn(t15, -1.0f / 3.0f));
     // extents and centre offsets from the exact box and COM
     double hm = 0.0, d2 = 0.0;
     const double com[3] = {r.cx, r.cy, r.cz};
+#pragma unroll
     for (int k = 0; k < 3; k++) {
       const double v = 0.5 * ((double)bmax[k] + (double)bmin[k]) - com[k];
       hm = fmax(hm, 0.5 * ((double)bmax[k] - (double)bmin[k]));
@@ -96,147 +91,231 @@ __device__ __forceinline__ void store_cell(int c, const MpRec& r, const typename
     l = fmaxf(__fmul_rn(2.0f, fmaxf(hx, fmaxf(hy, hz))), 1.0e-6f);
   }
   const float op = __fmaf_rn(l, inv_theta, s);
-  cell_open[c] = make_float4(cx, cy, cz, __fmul_rn(op, op));
+  q.open = make_float4(cx, cy, cz, __fmul_rn(op, op));
   // per-group opening angles recompute (l/theta_g + s)^2; the relative test
   // compares M l^3 (formed once here, in float) with tau ds^5
   const float mf = (float)r.m;
-  const double tr = r.ixx + r.iyy + r.izz;
-  const float t15 = (float)(1.5 * tr);
   // (the relative test's size is the box's l: the mass-weighted rms radius
   // sqrt(tr I / M) in its place ran 3-4 % slower at equal median error)
   const float mk = __fmul_rn(mf, __fmul_rn(l, __fmul_rn(l, l)));
-  cell_ls[c] = make_float4(l, s, mk, t15);
+  q.ls = make_float4(l, s, mk, t15);
   // the walk's staged record, copied to shared memory as it is (moments
   // negated so that every difference in the interaction is one add)
-  float4* st = cell_stage + 3 * (size_t)c;
-  st[0] = make_float4(cx, cy, cz, __fmul_rn(t15, -1.0f / 3.0f));
-  st[1] = make_float4(mf, -(float)(3.0 * r.ixx), -(float)(3.0 * r.iyy), -(float)(3.0 * r.izz));
-  st[2] = make_float4(-(float)(3.0 * r.ixy), -(float)(3.0 * r.ixz), -(float)(3.0 * r.iyz), -t15);
+  q.stage[0] = make_float4(cx, cy, cz, __fmul_rn(t15, -1.0f / 3.0f));
+  q.stage[1] = make_float4(mf, -(float)(3.0 * r.ixx), -(float)(3.0 * r.iyy), -(float)(3.0 * r.izz));
+  q.stage[2] = make_float4(-(float)(3.0 * r.ixy), -(float)(3.0 * r.ixz), -(float)(3.0 * r.iyz), -t15);
+  return q;
 }
 
-// A child's record fields (written by an earlier launch): 16-byte vector loads
-// through L1, so a record costs 5 load instructions and its second read hits
-// L1.
-__device__ __forceinline__ void load_mass_com(const MpRec* r, double& m, double& x, double& y, double& z) {
-  const double2 a = __ldg(reinterpret_cast<const double2*>(r)), b = __ldg(reinterpret_cast<const double2*>(r) + 1);
-  m = a.x; x = a.y; y = b.x; z = b.y;
+// box of cell c as two-element vectors (24 or 48 bytes per cell)
+__device__ __forceinline__ void store_box(float* box, int c, const float* lo, const float* hi) {
+  float2* b = reinterpret_cast<float2*>(box + 6 * (size_t)c);
+  b[0] = make_float2(lo[0], lo[1]); b[1] = make_float2(lo[2], hi[0]); b[2] = make_float2(hi[1], hi[2]);
 }
-__device__ __forceinline__ MpRec load_rec(const MpRec* r) {
-  MpRec o;
-  const double2* q = reinterpret_cast<const double2*>(r);
-  const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3), e = __ldg(q + 4);
-  o.m = a.x; o.cx = a.y; o.cy = b.x; o.cz = b.y;
-  o.ixx = c.x; o.iyy = c.y; o.izz = d.x; o.ixy = d.y; o.ixz = e.x; o.iyz = e.y;
-  return o;
+__device__ __forceinline__ void store_box(double* box, int c, const double* lo, const double* hi) {
+  double2* b = reinterpret_cast<double2*>(box + 6 * (size_t)c);
+  b[0] = make_double2(lo[0], lo[1]); b[1] = make_double2(lo[2], hi[0]); b[2] = make_double2(hi[1], hi[2]);
 }
-__device__ __forceinline__ void load_box(const float* bk, float lo[3], float hi[3]) {
-  const float2* q = reinterpret_cast<const float2*>(bk);  // 24 B per cell: 8-byte aligned
-  const float2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-  lo[0] = a.x; lo[1] = a.y; lo[2] = b.x; hi[0] = b.y; hi[1] = c.x; hi[2] = c.y;
+__device__ __forceinline__ void load_box(const float* box, int c, float* lo, float* hi) {
+  const float2* q = reinterpret_cast<const float2*>(box + 6 * (size_t)c);
+  const float2 a = __ldcg(q), b = __ldcg(q + 1), d = __ldcg(q + 2);
+  lo[0] = a.x; lo[1] = a.y; lo[2] = b.x; hi[0] = b.y; hi[1] = d.x; hi[2] = d.y;
 }
-__device__ __forceinline__ void load_box(const double* bk, double lo[3], double hi[3]) {
-  const double2* q = reinterpret_cast<const double2*>(bk);  // 48 B per cell: 16-byte aligned
-  const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-  lo[0] = a.x; lo[1] = a.y; lo[2] = b.x; hi[0] = b.y; hi[1] = c.x; hi[2] = c.y;
+__device__ __forceinline__ void load_box(const double* box, int c, double* lo, double* hi) {
+  const double2* q = reinterpret_cast<const double2*>(box + 6 * (size_t)c);
+  const double2 a = __ldcg(q), b = __ldcg(q + 1), d = __ldcg(q + 2);
+  lo[0] = a.x; lo[1] = a.y; lo[2] = b.x; hi[0] = b.y; hi[1] = d.x; hi[2] = d.y;
 }
 
-// A parent's moments from its nch contiguous children (parallel-axis
-// theorem, FP64), the children taken in index order.
-template <bool DS>
-__device__ void combine_children(int p, int first, int nch, float inv_theta, MpRec* __restrict__ rec,
-                                 typename BoxOf<DS>::T* __restrict__ box, float4* __restrict__ cell_open,
-                                 float4* __restrict__ cell_stage,
-                                 float4* __restrict__ cell_ls, float4* __restrict__ cell_lo) {
-  typedef typename BoxOf<DS>::T B;
-  double M = 0, X = 0, Y = 0, Z = 0;
-  B bmn[3] = {(B)3.0e38, (B)3.0e38, (B)3.0e38}, bmx[3] = {(B)-3.0e38, (B)-3.0e38, (B)-3.0e38};
-  // the children's records are loaded a batch ahead of their sums, which
-  // stay in child order (the moments are the same to the bit)
-  constexpr int kB = 4;
-  for (int k0 = 0; k0 < nch; k0 += kB) {
-    double mb[kB], xb[kB], yb[kB], zb[kB];
-    B lo[kB][3], hi[kB][3];
-#pragma unroll
-    for (int u = 0; u < kB; u++) {
-      const int k = min(k0 + u, nch - 1);
-      load_mass_com(rec + first + k, mb[u], xb[u], yb[u], zb[u]);
-      load_box(box + 6 * (size_t)(first + k), lo[u], hi[u]);
+// ---------------------------------------------------------------------------
+// Nodes, all levels in one cooperative launch: a grid-wide barrier between
+// levels, eight lanes per node, one per child.  The records of a node's
+// contiguous children are copied to shared memory by consecutive 16-byte
+// loads; lanes then hold either a child (its parallel-axis terms) or a
+// quantity (its sum over the children in child order), so a node costs about
+// three memory round trips and the sums keep their order.  Bound by the
+// levels' latency (about 2.5 us a level) below a million particles and by
+// record traffic above.  Against one launch per level and one thread per node,
+// 20 launches: 1024 particles 57 -> 17 us, 30,011 73 -> 33, 250,007 (leaves of 8)
+// 111 -> 75, 2^20 117 -> 99; 2^24 363 -> 416 beside the group branch's gather
+// (the whole step is the same there).
+// ---------------------------------------------------------------------------
+constexpr int kLvThreads = 512;
+constexpr int kLvWarps = kLvThreads / 32;
+constexpr int kLvMaxBlocksPerSm = 2;
+// a node's eight child records in shared memory (doubles): 81, so that the two
+// nodes of a half-warp fall on other banks
+constexpr int kNodeDoubles = 81;
+constexpr int kNarrow = 256;  // cells of a level that one block takes (64 teams)
+constexpr int kBarrierSpin = 1 << 24;
+
+// All blocks have arrived `round` times.  The wait is bounded: past the bound
+// it reports, and the caller returns (results invalid).
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned round, int* status) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(count, 1u);
+    const unsigned target = round * gridDim.x;
+    volatile unsigned* c = count;
+    int spin = 0;
+    while (*c < target && spin < kBarrierSpin) {
+      __nanosleep(20);
+      spin++;
     }
+    ok = *c >= target;
+    if (!ok) set_status(status, kStatusSortTimeout);
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+template <bool DS>
+__global__ void __launch_bounds__(kLvThreads, kLvMaxBlocksPerSm)
+    k_mp_levels(TreeInfo* __restrict__ info, const uint4* __restrict__ cell_data, float inv_theta, MpRec* rec,
+                typename BoxOf<DS>::T* box, float4* __restrict__ cell_open, float4* __restrict__ cell_stage,
+                float4* __restrict__ cell_ls, int cell_cap, float4* __restrict__ cell_lo, unsigned* barrier) {
+  typedef typename BoxOf<DS>::T B;
+  extern __shared__ double node_sm[];
+  const int ncells = info->ncells;
+  if (ncells > cell_cap) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, team = lane >> 3, t = lane & 7;
+  double* sm = node_sm + (size_t)(w * 4 + team) * kNodeDoubles;
+  const int nwarps = gridDim.x * kLvWarps, gw = blockIdx.x * kLvWarps + w;
+  unsigned round = 0;
+  const int top = info->nlevels - 1;
+  for (int L = top; L >= 1; L--) {
+    const int b = info->level_beg[L], e = info->level_end[L];
+    // A narrow level is the first block's alone, and between two narrow levels
+    // the block's own barrier will do: a grid-wide one, about as long as the
+    // level itself, is taken only before a wide level and after it.
+    const bool narrow = e - b <= kNarrow;
+    // cells a warp looks at together: fewer where the level would leave warps idle
+    const int nw = narrow ? kLvWarps : nwarps;
+    int span = 4;
+    while (span < 32 && (long long)span * nw < e - b) span *= 2;
+    const int cfirst = b + gw * span;
+    // the first cells' words do not wait for the level below
+    unsigned yl = (lane < span && cfirst + lane < e) ? __ldg(&cell_data[cfirst + lane].y) : 0xFFFFFFFFu;
+    if (L < top) {
+      const bool below = info->level_end[L + 1] - info->level_beg[L + 1] <= kNarrow;
+      if (narrow && below) __syncthreads();
+      else if (!grid_barrier(barrier, ++round, &info->status)) return;
+    }
+    if (narrow && blockIdx.x != 0) continue;
+    for (int c0 = cfirst; c0 < e; c0 += nw * span) {
+      if (c0 != cfirst) yl = (lane < span && c0 + lane < e) ? __ldg(&cell_data[c0 + lane].y) : 0xFFFFFFFFu;
+      unsigned nodes = __ballot_sync(kFull, yl != 0xFFFFFFFFu);
+      while (nodes) {
+        // this team's node: the team-th of the remaining ones
+        unsigned rest = nodes;
+        for (int k = 0; k < team; k++) rest &= rest - 1;
+        const int src = rest ? __ffs(rest) - 1 : 0;
+        const unsigned y = __shfl_sync(kFull, yl, src);
+        const int p = c0 + src;
+        const int first = (int)(y & 0x1FFFFFFFu);
+        int nch = rest ? (int)(y >> 29) + 1 : 0;
+        if (nch && !BONSAI_IN_RANGE(first + nch - 1, ncells, 0x307)) nch = 0;
+        for (int k = 0; k < 4 && nodes; k++) nodes &= nodes - 1;
+        // the children's records, 5 x 16 bytes each, and this lane's child's box
+        const double2* src2 = reinterpret_cast<const double2*>(rec + first);
+        double2 v[5];
 #pragma unroll
-    for (int u = 0; u < kB; u++) {
-      if (k0 + u >= nch) break;
-      const double mk = mb[u];
-      M += mk;
-      X += mk * xb[u]; Y += mk * yb[u]; Z += mk * zb[u];
+        for (int k = 0; k < 5; k++)
+          if (t + 8 * k < 5 * nch) v[k] = __ldcg(src2 + t + 8 * k);
+        B lo[3], hi[3];
+        if (t < nch) {
+          load_box(box, first + t, lo, hi);
+        } else {
 #pragma unroll
-      for (int a = 0; a < 3; a++) {
-        bmn[a] = DS ? (B)fmin((double)bmn[a], (double)lo[u][a]) : (B)fminf((float)bmn[a], (float)lo[u][a]);
-        bmx[a] = DS ? (B)fmax((double)bmx[a], (double)hi[u][a]) : (B)fmaxf((float)bmx[a], (float)hi[u][a]);
+          for (int a = 0; a < 3; a++) { lo[a] = (B)3.0e38; hi[a] = (B)-3.0e38; }
+        }
+#pragma unroll
+        for (int k = 0; k < 5; k++)
+          if (t + 8 * k < 5 * nch) {
+            sm[2 * (t + 8 * k)] = v[k].x;
+            sm[2 * (t + 8 * k) + 1] = v[k].y;
+          }
+#pragma unroll
+        for (int o = 4; o; o >>= 1)
+#pragma unroll
+          for (int a = 0; a < 3; a++) {
+            const B x = __shfl_xor_sync(kFull, lo[a], o), z = __shfl_xor_sync(kFull, hi[a], o);
+            lo[a] = DS ? (B)fmin((double)lo[a], (double)x) : (B)fminf((float)lo[a], (float)x);
+            hi[a] = DS ? (B)fmax((double)hi[a], (double)z) : (B)fmaxf((float)hi[a], (float)z);
+          }
+        __syncwarp();
+        // lanes 0..3: M and the mass-weighted coordinates, in child order
+        double sum = 0.0;
+#pragma unroll 4
+        for (int k = 0; k < nch; k++) sum = fma(sm[10 * k], (t & 3) ? sm[10 * k + (t & 3)] : 1.0, sum);
+        MpRec P;
+        P.m = __shfl_sync(kFull, sum, team * 8);
+        double com = P.m > 0.0 ? sum / P.m : 0.0;
+        if (!(P.m > 0.0) && (t & 3)) {
+          const int a = (t & 3) - 1;
+          com = 0.5 * ((double)(a == 0 ? lo[0] : a == 1 ? lo[1] : lo[2]) + (a == 0 ? hi[0] : a == 1 ? hi[1] : hi[2]));
+        }
+        P.cx = __shfl_sync(kFull, com, team * 8 + 1);
+        P.cy = __shfl_sync(kFull, com, team * 8 + 2);
+        P.cz = __shfl_sync(kFull, com, team * 8 + 3);
+        // each lane its child's terms about the new centre, into the child's slots
+        if (t < nch) {
+          double* q = sm + 10 * t;
+          const double mk = q[0];
+          const double dx = q[1] - P.cx, dy = q[2] - P.cy, dz = q[3] - P.cz;
+          q[4] = q[4] + mk * dx * dx;
+          q[5] = q[5] + mk * dy * dy;
+          q[6] = q[6] + mk * dz * dz;
+          q[7] = q[7] + mk * dx * dy;
+          q[8] = q[8] + mk * dx * dz;
+          q[9] = q[9] + mk * dy * dz;
+        }
+        __syncwarp();
+        // lanes 0..5: one moment each, in child order
+        double in = 0.0;
+        if (t < 6) {
+#pragma unroll 4
+          for (int k = 0; k < nch; k++) in += sm[10 * k + 4 + t];
+        }
+        P.ixx = __shfl_sync(kFull, in, team * 8);
+        P.iyy = __shfl_sync(kFull, in, team * 8 + 1);
+        P.izz = __shfl_sync(kFull, in, team * 8 + 2);
+        P.ixy = __shfl_sync(kFull, in, team * 8 + 3);
+        P.ixz = __shfl_sync(kFull, in, team * 8 + 4);
+        P.iyz = __shfl_sync(kFull, in, team * 8 + 5);
+        if (nch) {
+          // the lanes share the stores
+          const CellOut q = cell_out<DS>(P, lo, hi, inv_theta);
+          double2* rp = reinterpret_cast<double2*>(rec + p);
+          if (t == 0) { rp[0] = make_double2(P.m, P.cx); cell_open[p] = q.open; }
+          if (t == 1) { rp[1] = make_double2(P.cy, P.cz); cell_ls[p] = q.ls; }
+          if (t == 2) { rp[2] = make_double2(P.ixx, P.iyy); cell_stage[3 * (size_t)p] = q.stage[0]; }
+          if (t == 3) { rp[3] = make_double2(P.izz, P.ixy); cell_stage[3 * (size_t)p + 1] = q.stage[1]; }
+          if (t == 4) { rp[4] = make_double2(P.ixz, P.iyz); cell_stage[3 * (size_t)p + 2] = q.stage[2]; }
+          if (t == 5) store_box(box, p, lo, hi);
+          if (DS && t == 6) cell_lo[p] = q.lo;
+        }
+        __syncwarp();  // the shared records are free for the next nodes
       }
     }
-  }
-  MpRec P;
-  if (M > 0.0) { P.cx = X / M; P.cy = Y / M; P.cz = Z / M; }
-  else {
-    P.cx = 0.5 * ((double)bmn[0] + bmx[0]); P.cy = 0.5 * ((double)bmn[1] + bmx[1]);
-    P.cz = 0.5 * ((double)bmn[2] + bmx[2]);
-  }
-  double I[6] = {0, 0, 0, 0, 0, 0};
-  constexpr int kB2 = 2;
-  for (int k0 = 0; k0 < nch; k0 += kB2) {
-    MpRec cb[kB2];
-#pragma unroll
-    for (int u = 0; u < kB2; u++) {
-      cb[u] = load_rec(rec + first + min(k0 + u, nch - 1));
-    }
-#pragma unroll
-    for (int u = 0; u < kB2; u++) {
-      if (k0 + u >= nch) break;
-      const double mk = cb[u].m;
-      const double dx = cb[u].cx - P.cx, dy = cb[u].cy - P.cy, dz = cb[u].cz - P.cz;
-      I[0] += cb[u].ixx + mk * dx * dx;
-      I[1] += cb[u].iyy + mk * dy * dy;
-      I[2] += cb[u].izz + mk * dz * dz;
-      I[3] += cb[u].ixy + mk * dx * dy;
-      I[4] += cb[u].ixz + mk * dx * dz;
-      I[5] += cb[u].iyz + mk * dy * dz;
-    }
-  }
-  P.m = M;
-  P.ixx = I[0]; P.iyy = I[1]; P.izz = I[2]; P.ixy = I[3]; P.ixz = I[4]; P.iyz = I[5];
-  store_cell<DS>(p, P, bmn, bmx, inv_theta, rec, box, cell_open, cell_stage, cell_ls, cell_lo);
-}
-
-// The nodes of one level from their children, one thread per cell (leaves
-// were done by the leaf pass).
-template <bool DS>
-__global__ void __launch_bounds__(256, BONSAI_MP_MINB) k_mp_level(int L, const TreeInfo* __restrict__ info,
-                                                  const uint4* __restrict__ cell_data, float inv_theta,
-                                                  MpRec* __restrict__ rec, typename BoxOf<DS>::T* __restrict__ box,
-                                                  float4* __restrict__ cell_open, float4* __restrict__ cell_stage, float4* __restrict__ cell_ls,
-                                                  int cell_cap, float4* __restrict__ cell_lo) {
-  if (info->ncells > cell_cap) return;
-  [[maybe_unused]] const int ncells = info->ncells;
-  const int b = info->level_beg[L], e = info->level_end[L];
-  for (int c = b + blockIdx.x * blockDim.x + threadIdx.x; c < e; c += gridDim.x * blockDim.x) {
-    const unsigned y = cell_data[c].y;
-    if (y == 0xFFFFFFFFu) continue;
-    const int first = (int)(y & 0x1FFFFFFFu), nch = (int)(y >> 29) + 1;
-    if (!BONSAI_IN_RANGE(first + nch - 1, ncells, 0x307)) continue;
-    combine_children<DS>(c, first, nch, inv_theta, rec, box, cell_open, cell_stage, cell_ls, cell_lo);
   }
 }
 
 // One thread per leaf: the leaf's moments (one pass by default).
 template <bool DS>
-__global__ void __launch_bounds__(256, BONSAI_MP_MINB) k_multipoles(const int* __restrict__ leaf_list, const TreeInfo* __restrict__ info,
+__global__ void __launch_bounds__(256) k_multipoles(const int* __restrict__ leaf_list, const TreeInfo* __restrict__ info,
                                                     const uint4* __restrict__ cell_data,
                                                     const float4* __restrict__ jpos, float inv_theta,
                                                     MpRec* __restrict__ rec, typename BoxOf<DS>::T* __restrict__ box,
                                                     float4* __restrict__ cell_open, float4* __restrict__ cell_stage, float4* __restrict__ cell_ls,
                                                     int cell_cap,
-                                                    const float4* __restrict__ jlo, float4* __restrict__ cell_lo) {
+                                                    const float4* __restrict__ jlo, float4* __restrict__ cell_lo,
+                                                    unsigned* __restrict__ barrier) {
   typedef typename BoxOf<DS>::T B;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *barrier = 0u;  // of the level launch that follows
   const int nleaves = info->nleaves;
   if (info->ncells > cell_cap) return;
   [[maybe_unused]] const int ncells = info->ncells, npart = info->npart;
@@ -336,30 +415,59 @@ __global__ void __launch_bounds__(256, BONSAI_MP_MINB) k_multipoles(const int* _
 #endif
     r.m = m;
     r.ixx = q[0]; r.iyy = q[1]; r.izz = q[2]; r.ixy = q[3]; r.ixz = q[4]; r.iyz = q[5];
-    store_cell<DS>(c, r, mn, mx, inv_theta, rec, box, cell_open, cell_stage, cell_ls, cell_lo);
+    const CellOut o = cell_out<DS>(r, mn, mx, inv_theta);
+    double2* rp = reinterpret_cast<double2*>(rec + c);
+    rp[0] = make_double2(r.m, r.cx);
+    rp[1] = make_double2(r.cy, r.cz);
+    rp[2] = make_double2(r.ixx, r.iyy);
+    rp[3] = make_double2(r.izz, r.ixy);
+    rp[4] = make_double2(r.ixz, r.iyz);
+    store_box(box, c, mn, mx);
+    cell_open[c] = o.open;
+    cell_ls[c] = o.ls;
+    for (int k = 0; k < 3; k++) cell_stage[3 * (size_t)c + k] = o.stage[k];
+    if (DS) cell_lo[c] = o.lo;
   }
 }
 
-void launch_multipoles(const int* leaf_list, const TreeInfo* info, const uint4* cell_data, const float4* jpos,
+constexpr int kLvSmem = kLvWarps * 4 * kNodeDoubles * (int)sizeof(double);
+
+// blocks of the level launch that are resident at once
+int multipole_level_blocks(int nsm) {
+  int a = 0, b = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_mp_levels<false>, kLvThreads, kLvSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_mp_levels<true>, kLvThreads, kLvSmem) != cudaSuccess)
+    return 1;
+  return std::max(1, nsm * std::min(std::min(a, b), kLvMaxBlocksPerSm));
+}
+
+template <bool DS>
+static void launch_multipoles_of(const int* leaf_list, TreeInfo* info, const uint4* cell_data, const float4* jpos,
+                                 int n, float inv_theta, MpRec* rec, typename BoxOf<DS>::T* box, float4* cell_open,
+                                 float4* cell_stage, float4* cell_ls, int cell_cap, const float4* jlo,
+                                 float4* cell_lo, int nblocks, unsigned* barrier, int level_blocks, cudaStream_t s) {
+  k_multipoles<DS><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, jpos, inv_theta, rec, box, cell_open,
+                                           cell_stage, cell_ls, cell_cap, jlo, cell_lo, barrier);
+  // about 1024 particles per block: more give the widest level its teams, fewer
+  // make the barrier cheaper
+  int grid = std::min(level_blocks, std::max(1, n / 1024));
+  void* args[] = {&info, &cell_data, &inv_theta, &rec, &box, &cell_open, &cell_stage, &cell_ls, &cell_cap, &cell_lo,
+                  &barrier};
+  cudaLaunchCooperativeKernel((const void*)k_mp_levels<DS>, dim3(grid), dim3(kLvThreads), args, (size_t)kLvSmem, s);
+}
+
+void launch_multipoles(const int* leaf_list, TreeInfo* info, const uint4* cell_data, const float4* jpos, int n,
                        float inv_theta, MpRec* rec, void* box, float4* cell_open, float4* cell_stage,
                        float4* cell_ls, int cell_cap, const float4* jlo, float4* cell_lo, int nblocks,
-                       cudaStream_t s) {
-  // leaves, then the nodes level by level from the deepest (levels 20 .. 1)
-  if (jlo) {
-    k_multipoles<true><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, jpos, inv_theta, rec,
-                                               static_cast<double*>(box), cell_open, cell_stage, cell_ls, cell_cap,
-                                               jlo, cell_lo);
-    for (int L = kMaxLevel - 1; L >= 1; L--)
-      k_mp_level<true><<<nblocks, 256, 0, s>>>(L, info, cell_data, inv_theta, rec, static_cast<double*>(box),
-                                               cell_open, cell_stage, cell_ls, cell_cap, cell_lo);
-  } else {
-    k_multipoles<false><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, jpos, inv_theta, rec,
-                                                static_cast<float*>(box), cell_open, cell_stage, cell_ls, cell_cap,
-                                                nullptr, nullptr);
-    for (int L = kMaxLevel - 1; L >= 1; L--)
-      k_mp_level<false><<<nblocks, 256, 0, s>>>(L, info, cell_data, inv_theta, rec, static_cast<float*>(box),
-                                                cell_open, cell_stage, cell_ls, cell_cap, nullptr);
-  }
+                       unsigned* barrier, int level_blocks, cudaStream_t s) {
+  if (jlo)
+    launch_multipoles_of<true>(leaf_list, info, cell_data, jpos, n, inv_theta, rec, static_cast<double*>(box),
+                               cell_open, cell_stage, cell_ls, cell_cap, jlo, cell_lo, nblocks, barrier,
+                               level_blocks, s);
+  else
+    launch_multipoles_of<false>(leaf_list, info, cell_data, jpos, n, inv_theta, rec, static_cast<float*>(box),
+                                cell_open, cell_stage, cell_ls, cell_cap, nullptr, nullptr, nblocks, barrier,
+                                level_blocks, s);
 }
 
 // Reference-layout view of the multipoles (debug/parity getter):

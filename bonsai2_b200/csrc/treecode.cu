@@ -109,6 +109,8 @@ struct Handle {
   unsigned long long* stats = nullptr;
   double *move_partial = nullptr, *energies = nullptr;
   unsigned *move_ticket = nullptr, *box_ticket = nullptr;
+  unsigned* mp_barrier = nullptr;  // of the multipoles' level launch
+  int mp_level_blocks = 1;
   int* closing = nullptr;
   Box* box = nullptr;
   float* box_partial = nullptr;
@@ -263,7 +265,7 @@ struct Handle {
     release_particles();
     dfree(&info); dfree(&g_count); dfree(&g_seg); dfree(&g_ng); dfree(&ring);
     dfree(&group_counter); dfree(&stats); dfree(&move_partial); dfree(&energies);
-    dfree(&move_ticket); dfree(&box_ticket); dfree(&closing); dfree(&acc_valid); dfree(&box); dfree(&box_partial);
+    dfree(&move_ticket); dfree(&box_ticket); dfree(&mp_barrier); dfree(&closing); dfree(&acc_valid); dfree(&box); dfree(&box_partial);
     dfree(&ph_table); dfree(&direct_part); dfree(&direct_out); dfree(&direct_sample);
     dfree(&mlp_w);
     if (mlp_wh) { cudaFree(mlp_wh); mlp_wh = nullptr; }
@@ -334,6 +336,8 @@ struct Handle {
     BONSAI_CUDA_TRY(cudaMemset(energies, 0, 8 * sizeof(double)));
     BONSAI_CUDA_TRY(dalloc(&move_ticket, 1));
     BONSAI_CUDA_TRY(dalloc(&box_ticket, 1));
+    BONSAI_CUDA_TRY(dalloc(&mp_barrier, 1));
+    mp_level_blocks = multipole_level_blocks(nsm);
     BONSAI_CUDA_TRY(cudaMemset(move_ticket, 0, sizeof(unsigned)));
     BONSAI_CUDA_TRY(cudaMemset(box_ticket, 0, sizeof(unsigned)));
     BONSAI_CUDA_TRY(dalloc(&closing, 1));
@@ -492,8 +496,9 @@ struct Handle {
                so(), nsys, root_beg, st);
   }
   void enq_multipoles() {
-    launch_multipoles(leaf_list, info, cell_data, jpos, 1.0f / prm.theta, rec, cell_box, cell_open, cell_stage,
-                      cell_ls, cap_cells, precision ? jlo : nullptr, precision ? cell_lo : nullptr, nsm * 8, st);
+    launch_multipoles(leaf_list, info, cell_data, jpos, n, 1.0f / prm.theta, rec, cell_box, cell_open, cell_stage,
+                      cell_ls, cap_cells, precision ? jlo : nullptr, precision ? cell_lo : nullptr, nsm * 8,
+                      mp_barrier, mp_level_blocks, st);
   }
   void enq_groups(int ls, int ncrit) { enq_groups_on(ls, ncrit, st, kalt, valt, sort_counts); }
   void enq_groups_on(int ls, int ncrit, cudaStream_t s, unsigned long long* ka, int* va, unsigned* work) {
