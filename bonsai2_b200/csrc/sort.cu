@@ -5,23 +5,34 @@
 // makeGroups.cu:270-277, buildTree.cu:940-944): a stable radix sort, ties in
 // input order.  This is a hand-written replacement with the same semantics:
 // 8 passes of 8 bits, one-sweep (below): keys are ranked stably inside each
-// 4096-key tile (the lanes of equal digit from bit ballots) with per-warp
+// tile (the lanes of equal digit from bit ballots) with per-warp
 // digit counters in shared memory, tile offsets come from a decoupled look-back, and tiles are written
 // out through shared memory in contiguous digit runs.  A thread keeps only the
-// 16 ranks and packed digits of its keys across the look-back (the keys are
+// ranks and packed digits of its keys across the look-back (the keys are
 // re-read from L2 for staging): 4 blocks per SM (keeping the keys, 127
 // registers and 2 blocks per SM, was 16 % slower per sort than 3 blocks).
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
 namespace bonsai {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096
 constexpr int kScanChunk = 4096;
+// Keys per thread of a one-sweep tile: 4 (1024-key tiles) while one wave of
+// tiles holds all keys, where a pass is one tile's latency (30,011 keys: 6.1 us
+// against 11); 16 above, where the digit runs that a tile writes out are longer
+// (2^20 keys, two sorts at once: 27 us either way; more tiles mean more look-back
+// words).  Same order either way.
+constexpr int kSmallItems = 4, kLargeItems = 16;
+constexpr int kSortSmallMax = 1 << 19;
+static int sort_items(int n) { return n <= kSortSmallMax ? kSmallItems : kLargeItems; }
 
-int sort_tiles(int n) { return (n + kSortTile - 1) / kSortTile; }
+int sort_tiles(int n) {
+  const int tile = kSortThreads * sort_items(n);
+  return (n + tile - 1) / tile;
+}
 
 // ---------------------------------------------------------------------------
 // exclusive scan of unsigned ints (length m known on the host)
@@ -130,26 +141,17 @@ void exclusive_scan(const unsigned* in, unsigned* out, int m, unsigned* bsum, un
 #endif
 constexpr unsigned kFlagAgg = 1u << 30, kFlagInc = 2u << 30, kValMask = (1u << 30) - 1u;
 
-// The lanes holding the same digit (0..256, 256 = no key): the intersection
-// of nine bit ballots (BONSAI_SORT_BALLOT_MATCH, the default), or
-// __match_any_sync, which was slower on the B200 (PH sort + group formation at
-// N = 2^24: 1.82 against 1.93 ms).  Issuing all items' ballots before the
-// chain through the warp's counters was measured no faster.
-#ifndef BONSAI_SORT_BALLOT_MATCH
-#define BONSAI_SORT_BALLOT_MATCH 1
-#endif
-__device__ __forceinline__ unsigned digit_peers(unsigned d) {
-#if BONSAI_SORT_BALLOT_MATCH
-  unsigned m = kFull;
+// The lanes of `live` that hold the same digit (0..255): the intersection of
+// eight bit ballots (__match_any_sync was slower on the B200: PH sort + group
+// formation at N = 2^24 1.93 against 1.82 ms).
+__device__ __forceinline__ unsigned digit_peers(unsigned d, unsigned live) {
+  unsigned m = live;
 #pragma unroll
-  for (int b = 0; b < 9; b++) {
+  for (int b = 0; b < 8; b++) {
     const unsigned bal = __ballot_sync(kFull, (d >> b) & 1u);
     m &= ((d >> b) & 1u) ? bal : ~bal;
   }
   return m;
-#else
-  return __match_any_sync(kFull, d);
-#endif
 }
 constexpr int kLookbackSpin = 1 << 22;
 
@@ -171,31 +173,35 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_hist8(const unsigned long
   }
 }
 
-// exclusive scan of each 256-entry row in place (one block, 256 threads)
-__global__ void __launch_bounds__(256) k_sort_hist_scan(unsigned* __restrict__ ghist, int passes) {
+// exclusive scan of each 256-entry row in place (one block of 256 threads per row)
+__global__ void __launch_bounds__(256) k_sort_hist_scan(unsigned* __restrict__ ghist) {
   __shared__ unsigned sh[32];
-  for (int p = 0; p < passes; p++) {
-    const unsigned v = ghist[p * 256 + threadIdx.x];
-    const unsigned e = block_excl_scan(v, sh, nullptr);
-    ghist[p * 256 + threadIdx.x] = e;
-    __syncthreads();
-  }
+  unsigned* row = ghist + blockIdx.x * 256;
+  const unsigned e = block_excl_scan(row[threadIdx.x], sh, nullptr);
+  row[threadIdx.x] = e;
 }
 
 // SYSD: the digit is a byte of the element's system index (sys_of of its
 // value, the element's position in the sort's input order), not of its key:
 // the passes that make an ensemble sort stable-partition by system last.
-template <bool SYSD>
+// The digits of all items are read before any is ranked: the ranking's warp
+// barriers would otherwise hold each load back behind the item before it, one
+// memory round trip per item (a pass over 30,011 keys 11.5 -> 6.1 us with the
+// smaller tiles).  The look-back reads four tiles' words at once (8 or 16 were no
+// faster below a million keys and slower above).
+constexpr int kLookback = 4;
+template <int ITEMS, bool SYSD>
 __global__ void __launch_bounds__(kSortThreads, BONSAI_SORT_MINB) k_sort_onesweep(
     const unsigned long long* __restrict__ keys_in, const int* __restrict__ vals_in, int n, int shift,
     const unsigned* __restrict__ gbase, unsigned* __restrict__ status, unsigned* __restrict__ tile_counter,
     unsigned long long* __restrict__ keys_out, int* __restrict__ vals_out, int* __restrict__ err,
     const int* __restrict__ sys_off, int nsys) {
+  constexpr int kTile = kSortThreads * ITEMS;
   __shared__ unsigned wcnt[kSortThreads / 32][256];
   __shared__ unsigned tile_off[256];
   __shared__ unsigned dstart[256];
-  __shared__ unsigned long long stage[kSortTile];  // keys, then values (as 32-bit) in digit order
-  __shared__ unsigned char sdig[kSortTile];
+  __shared__ unsigned long long stage[kTile];  // keys, then values (as 32-bit) in digit order
+  __shared__ unsigned char sdig[kTile];
   __shared__ unsigned sh[32];
   __shared__ int tile_sh;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -203,22 +209,26 @@ __global__ void __launch_bounds__(kSortThreads, BONSAI_SORT_MINB) k_sort_oneswee
   for (int t = threadIdx.x; t < (kSortThreads / 32) * 256; t += kSortThreads) (&wcnt[0][0])[t] = 0;
   __syncthreads();
   const int tile = tile_sh;
-  const int base = tile * kSortTile + w * (32 * kSortItems);
-  unsigned rank[kSortItems];
-  unsigned dpack[kSortItems / 4];
+  const int base = tile * kTile + w * (32 * ITEMS);
+  unsigned rank[ITEMS];
+  unsigned dpack[ITEMS / 4];
 #pragma unroll
-  for (int k = 0; k < kSortItems; k++) {
+  for (int k = 0; k < ITEMS; k++) {
     const int i = base + k * 32 + lane;
-    const bool ok = i < n;
-    unsigned d;
-    if constexpr (SYSD) {
-      d = ok ? (((unsigned)sys_of(sys_off, nsys, vals_in ? vals_in[i] : i) >> shift) & 255u) : 256u;
-    } else {
-      d = ok ? ((unsigned)(keys_in[i] >> shift) & 255u) : 256u;
+    unsigned d = 0u;
+    if (i < n) {
+      if constexpr (SYSD) d = ((unsigned)sys_of(sys_off, nsys, vals_in ? vals_in[i] : i) >> shift) & 255u;
+      else d = (unsigned)(keys_in[i] >> shift) & 255u;
     }
     if ((k & 3) == 0) dpack[k >> 2] = 0u;
-    dpack[k >> 2] |= (d & 255u) << (8 * (k & 3));
-    const unsigned peers = digit_peers(d);
+    dpack[k >> 2] |= d << (8 * (k & 3));
+  }
+#pragma unroll
+  for (int k = 0; k < ITEMS; k++) {
+    const bool ok = base + k * 32 + lane < n;
+    const unsigned live = __ballot_sync(kFull, ok);
+    const unsigned d = (dpack[k >> 2] >> (8 * (k & 3))) & 255u;
+    const unsigned peers = digit_peers(d, live);
     const unsigned before = (unsigned)__popc(peers & lanemask_lt());
     const unsigned cur = ok ? wcnt[w][d] : 0u;
     rank[k] = cur + before;
@@ -236,39 +246,43 @@ __global__ void __launch_bounds__(kSortThreads, BONSAI_SORT_MINB) k_sort_oneswee
     wcnt[ww][d] = tot;
     tot += c;
   }
+  volatile unsigned* st = status;
+  // published before the block's own scan: the tiles behind wait for it
+  st[(size_t)tile * 256 + d] = (tile == 0 ? kFlagInc : kFlagAgg) | tot;
   tile_off[d] = block_excl_scan(tot, sh, nullptr);
   // decoupled look-back for the digit's global offset
-  volatile unsigned* st = status;
-  if (tile == 0) {
-    st[d] = kFlagInc | tot;
-    dstart[d] = gbase[d];
-  } else {
-    st[(size_t)tile * 256 + d] = kFlagAgg | tot;
-    unsigned excl = 0;
-    for (int t = tile - 1; t >= 0; t--) {
-      unsigned v = st[(size_t)t * 256 + d];
+  unsigned excl = 0;
+  bool done = tile == 0;
+  for (int t = tile - 1; !done; t -= kLookback) {
+    unsigned v[kLookback];
+#pragma unroll
+    for (int q = 0; q < kLookback; q++) v[q] = t - q >= 0 ? (unsigned)st[(size_t)(t - q) * 256 + d] : (unsigned)kFlagInc;
+#pragma unroll
+    for (int q = 0; q < kLookback; q++) {
+      if (done) break;
       int spin = 0;
-      while ((v & ~kValMask) == 0u && spin < kLookbackSpin) {
+      while ((v[q] & ~kValMask) == 0u && spin < kLookbackSpin) {
         __nanosleep(32);
-        v = st[(size_t)t * 256 + d];
+        v[q] = st[(size_t)(t - q) * 256 + d];
         spin++;
       }
-      if ((v & ~kValMask) == 0u) {  // bound hit: report and give up (results invalid)
+      if ((v[q] & ~kValMask) == 0u) {  // bound hit: report and give up (results invalid)
         atomicOr(err, kStatusSortTimeout);
+        done = true;
         break;
       }
-      excl += v & kValMask;
-      if ((v & ~kValMask) == kFlagInc) break;
+      excl += v[q] & kValMask;
+      done = (v[q] & ~kValMask) == kFlagInc;
     }
-    st[(size_t)tile * 256 + d] = kFlagInc | (excl + tot);
-    dstart[d] = gbase[d] + excl;
   }
+  if (tile != 0) st[(size_t)tile * 256 + d] = kFlagInc | (excl + tot);
+  dstart[d] = gbase[d] + excl;
   __syncthreads();
   // stage keys in digit order (re-read from L2), write contiguous runs
-  const int tile_n = min(kSortTile, n - tile * kSortTile);
-  unsigned lpos[kSortItems];
+  const int tile_n = min(kTile, n - tile * kTile);
+  unsigned lpos[ITEMS];
 #pragma unroll
-  for (int k = 0; k < kSortItems; k++) {
+  for (int k = 0; k < ITEMS; k++) {
     const int i = base + k * 32 + lane;
     if (i < n) {
       const unsigned dd = (dpack[k >> 2] >> (8 * (k & 3))) & 255u;
@@ -287,7 +301,7 @@ __global__ void __launch_bounds__(kSortThreads, BONSAI_SORT_MINB) k_sort_oneswee
   __syncthreads();
   unsigned* stage32 = reinterpret_cast<unsigned*>(stage);
 #pragma unroll
-  for (int k = 0; k < kSortItems; k++) {
+  for (int k = 0; k < ITEMS; k++) {
     const int i = base + k * 32 + lane;
     if (i < n) stage32[lpos[k]] = (unsigned)(vals_in ? vals_in[i] : i);
   }
@@ -296,6 +310,103 @@ __global__ void __launch_bounds__(kSortThreads, BONSAI_SORT_MINB) k_sort_oneswee
     const unsigned dd = sdig[j];
     const unsigned dst = dstart[dd] + (unsigned)j - tile_off[dd];
     if (BONSAI_IN_RANGE(dst, n, 0x602)) vals_out[dst] = (int)stage32[j];
+  }
+}
+
+// All eight passes of at most 4096 keys in one block, the pairs in shared
+// memory throughout: a launch per pass is latency alone at this size (1024 keys:
+// 11.3 us for the whole sort, 8 launches of 7.2 us and two more before it).  Every
+// pass ranks as above: warp w's items are the 128 positions from 128 w.
+constexpr int kOneThreads = 1024, kOneItems = 4, kOneMax = kOneThreads * kOneItems;
+constexpr int kOneWarps = kOneThreads / 32;
+constexpr int kOneSmem = kOneMax * (8 + 4) + kOneWarps * 256 * 2 + 256 * 4;
+__global__ void __launch_bounds__(kOneThreads) k_sort_block(unsigned long long* __restrict__ keys,
+                                                            const int* __restrict__ vals_in,
+                                                            int* __restrict__ vals, int n, int passes) {
+  extern __shared__ unsigned long long one_sm[];
+  unsigned long long* sk = one_sm;
+  int* sv = reinterpret_cast<int*>(sk + kOneMax);
+  unsigned short* wc = reinterpret_cast<unsigned short*>(sv + kOneMax);  // [warp][digit]
+  unsigned* off = reinterpret_cast<unsigned*>(wc + kOneWarps * 256);     // digit offsets
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int base = w * 32 * kOneItems;
+  const int nw = (n + 32 * kOneItems - 1) / (32 * kOneItems);  // warps that hold keys
+  unsigned long long key[kOneItems];
+  int val[kOneItems];
+#pragma unroll
+  for (int k = 0; k < kOneItems; k++) {
+    const int i = base + 32 * k + lane;
+    key[k] = i < n ? keys[i] : 0ull;
+    val[k] = i < n ? (vals_in ? vals_in[i] : i) : 0;
+  }
+  for (int p = 0; p < passes; p++) {
+    for (int t = threadIdx.x; t < nw * 128; t += (int)blockDim.x) reinterpret_cast<unsigned*>(wc)[t] = 0u;
+    __syncthreads();
+    unsigned rank[kOneItems];
+#pragma unroll
+    for (int k = 0; k < kOneItems; k++) {
+      const bool ok = base + 32 * k + lane < n;
+      const unsigned live = __ballot_sync(kFull, ok);
+      const unsigned d = (unsigned)(key[k] >> (8 * p)) & 255u;
+      const unsigned peers = digit_peers(d, live);
+      const unsigned before = (unsigned)__popc(peers & lanemask_lt());
+      const unsigned cur = ok ? wc[w * 256 + d] : 0u;
+      rank[k] = cur + before;
+      __syncwarp();
+      if (ok && before == 0) wc[w * 256 + d] = (unsigned short)(cur + __popc(peers));
+      __syncwarp();
+    }
+    __syncthreads();
+    // a thread per digit: its counters become the prefix over the warps that
+    // hold keys
+    if (threadIdx.x < 256) {
+      const int d = threadIdx.x;
+      unsigned run = 0;
+#pragma unroll 8
+      for (int q = 0; q < nw; q++) {
+        const unsigned c = wc[q * 256 + d];
+        wc[q * 256 + d] = (unsigned short)run;
+        run += c;
+      }
+      off[d] = run;
+    }
+    __syncthreads();
+    if (w == 0) {
+      unsigned v[8], s = 0;
+#pragma unroll
+      for (int q = 0; q < 8; q++) { v[q] = off[lane * 8 + q]; s += v[q]; }
+      unsigned run = (unsigned)warp_incl_scan((int)s) - s;
+#pragma unroll
+      for (int q = 0; q < 8; q++) { off[lane * 8 + q] = run; run += v[q]; }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kOneItems; k++) {
+      if (base + 32 * k + lane < n) {
+        const unsigned d = (unsigned)(key[k] >> (8 * p)) & 255u;
+        const unsigned at = off[d] + wc[w * 256 + d] + rank[k];
+        sk[at] = key[k];
+        sv[at] = val[k];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kOneItems; k++) {
+      const int i = base + 32 * k + lane;
+      if (i < n) {
+        key[k] = sk[i];
+        val[k] = sv[i];
+      }
+    }
+    // (the next pass writes sk and sv only after three more barriers)
+  }
+#pragma unroll
+  for (int k = 0; k < kOneItems; k++) {
+    const int i = base + 32 * k + lane;
+    if (i < n) {
+      keys[i] = key[k];
+      vals[i] = val[k];
+    }
   }
 }
 
@@ -321,19 +432,22 @@ size_t sort_status_words(int n) { return (size_t)sort_tiles(n) * 256 * kMaxPasse
 // out as sys_off), two more passes order by system index, so each system's
 // pairs are sorted by key within the system's own index range, ties in input
 // order: the order each system gets when sorted alone.
-void radix_sort_pairs(unsigned long long* keys_a, unsigned long long* keys_b, int* vals_a, int* vals_b,
-                      const int* vals_in, int n, unsigned* work, int* err, int passes, const int* sys_off, int nsys,
-                      cudaStream_t s) {
-  if (n <= 0) return;
+template <int ITEMS>
+static void radix_sort_passes(unsigned long long* keys_a, unsigned long long* keys_b, int* vals_a, int* vals_b,
+                              const int* vals_in, int n, unsigned* work, int* err, int passes, const int* sys_off,
+                              int nsys, cudaStream_t s) {
   const int nt = sort_tiles(n);
   const int sys_passes = nsys > 1 ? 2 : 0;
-  unsigned* status = work;
-  unsigned* counters = work + (size_t)nt * 256 * kMaxPasses;
+  // counters, histograms, then the look-back words of the passes that run
+  unsigned* counters = work;
   unsigned* ghist = counters + kMaxPasses;
-  cudaMemsetAsync(work, 0, sort_status_words(n) * sizeof(unsigned), s);
-  k_sort_hist8<<<1184, kSortThreads, 0, s>>>(keys_a, n, passes, ghist);
+  unsigned* status = ghist + kMaxPasses * 256;
+  cudaMemsetAsync(work, 0, (kMaxPasses * 257 + (size_t)(passes + sys_passes) * nt * 256) * sizeof(unsigned), s);
+  // a block's histograms cost up to 2048 global atomics
+  const int per = n <= (1 << 17) ? 1024 : 4096;
+  k_sort_hist8<<<std::min((n + per - 1) / per, 1184), kSortThreads, 0, s>>>(keys_a, n, passes, ghist);
   if (sys_passes) k_sort_hist_sys<<<(nsys + 255) / 256, 256, 0, s>>>(sys_off, nsys, ghist + 256 * passes);
-  k_sort_hist_scan<<<1, 256, 0, s>>>(ghist, passes + sys_passes);
+  k_sort_hist_scan<<<passes + sys_passes, 256, 0, s>>>(ghist);
   unsigned long long* kin = keys_a;
   unsigned long long* kout = keys_b;
   int* vin = vals_a;
@@ -342,13 +456,29 @@ void radix_sort_pairs(unsigned long long* keys_a, unsigned long long* keys_b, in
     const int* vi = p == 0 ? vals_in : vin;
     unsigned* stp = status + (size_t)p * nt * 256;
     if (p < passes)
-      k_sort_onesweep<false><<<nt, kSortThreads, 0, s>>>(kin, vi, n, 8 * p, ghist + 256 * p, stp, counters + p, kout,
-                                                         vout, err, nullptr, 0);
+      k_sort_onesweep<ITEMS, false><<<nt, kSortThreads, 0, s>>>(kin, vi, n, 8 * p, ghist + 256 * p, stp,
+                                                                counters + p, kout, vout, err, nullptr, 0);
     else
-      k_sort_onesweep<true><<<nt, kSortThreads, 0, s>>>(kin, vi, n, 8 * (p - passes), ghist + 256 * p, stp,
-                                                        counters + p, kout, vout, err, sys_off, nsys);
+      k_sort_onesweep<ITEMS, true><<<nt, kSortThreads, 0, s>>>(kin, vi, n, 8 * (p - passes), ghist + 256 * p, stp,
+                                                               counters + p, kout, vout, err, sys_off, nsys);
     unsigned long long* tk = kin; kin = kout; kout = tk;
     int* tv = vin; vin = vout; vout = tv;
+  }
+}
+
+void radix_sort_pairs(unsigned long long* keys_a, unsigned long long* keys_b, int* vals_a, int* vals_b,
+                      const int* vals_in, int n, unsigned* work, int* err, int passes, const int* sys_off, int nsys,
+                      cudaStream_t s) {
+  if (n <= 0) return;
+  if (n <= kOneMax && nsys <= 1) {
+    cudaFuncSetAttribute(k_sort_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneSmem);
+    // the warps that hold keys, and a thread per digit
+    const int threads = std::max(256, (n + 32 * kOneItems - 1) / (32 * kOneItems) * 32);
+    k_sort_block<<<1, threads, kOneSmem, s>>>(keys_a, vals_in, vals_a, n, passes);
+  } else if (sort_items(n) == kSmallItems) {
+    radix_sort_passes<kSmallItems>(keys_a, keys_b, vals_a, vals_b, vals_in, n, work, err, passes, sys_off, nsys, s);
+  } else {
+    radix_sort_passes<kLargeItems>(keys_a, keys_b, vals_a, vals_b, vals_in, n, work, err, passes, sys_off, nsys, s);
   }
 }
 
@@ -358,7 +488,7 @@ void radix_sort_pairs(unsigned long long* keys_a, unsigned long long* keys_b, in
 // kStatusSortTimeout in *err, and tile 2 must then finish behind tile 1.
 // Returns the status bits (or a CUDA error as -1000 - code).
 int sort_timeout_selftest(cudaStream_t s) {
-  const int n = 3 * kSortTile, nt = 3;
+  const int n = 3 * kSortThreads * kLargeItems, nt = 3;
   unsigned long long *ka = nullptr, *kb = nullptr;
   int *va = nullptr, *err = nullptr;
   unsigned *status = nullptr, *counter = nullptr, *gbase = nullptr;
@@ -378,7 +508,7 @@ int sort_timeout_selftest(cudaStream_t s) {
     cudaMemsetAsync(err, 0, sizeof(int), s);
     const unsigned one = 1u;
     cudaMemcpyAsync(counter, &one, sizeof(unsigned), cudaMemcpyHostToDevice, s);
-    k_sort_onesweep<false><<<nt - 1, kSortThreads, 0, s>>>(ka, nullptr, n, 0, gbase, status, counter, kb, va + n, err,
+    k_sort_onesweep<kLargeItems, false><<<nt - 1, kSortThreads, 0, s>>>(ka, nullptr, n, 0, gbase, status, counter, kb, va + n, err,
                                                            nullptr, 0);
     cudaMemcpyAsync(&result, err, sizeof(int), cudaMemcpyDeviceToHost, s);
     e = cudaStreamSynchronize(s);
