@@ -41,6 +41,9 @@ __global__ void k_group_sizes(const unsigned* __restrict__ seg_beg, const unsign
     ng[b] = (seg_end[b] - seg_beg[b] + (unsigned)ncrit - 1u) / (unsigned)ncrit;
 }
 
+// order (optional): the groups in the order the walk takes them, those more than
+// half full from the front and the others from the back, so that the long ones
+// do not come last.
 // one thread per group: the group's bin is found by binary search over the
 // exclusive scan of group counts (bins near a dense core hold 10^5 groups, so
 // a thread per bin would serialise them)
@@ -48,7 +51,8 @@ __global__ void __launch_bounds__(256) k_group_write(const unsigned* __restrict_
                                                      const unsigned* __restrict__ seg_start,
                                                      const unsigned* __restrict__ goff, int nbins, int ncrit,
                                                      int2* __restrict__ groups, int group_cap,
-                                                     TreeInfo* __restrict__ info, [[maybe_unused]] int n) {
+                                                     TreeInfo* __restrict__ info, [[maybe_unused]] int n,
+                                                     int* __restrict__ order, unsigned* __restrict__ order_count) {
   const int ng = info->ngroups;
   if (ng > group_cap) {
     if (blockIdx.x == 0 && threadIdx.x == 0) set_status(&info->status, kStatusGroupCapacity);
@@ -67,21 +71,34 @@ __global__ void __launch_bounds__(256) k_group_write(const unsigned* __restrict_
     const int count = (int)(seg_end[lo] - seg_start[lo]);
     // every group holds at least one particle, inside the particle range
     if (!BONSAI_IN_RANGE(off, count, 0x203) || !BONSAI_IN_RANGE((int)seg_start[lo] + count - 1, n, 0x204)) continue;
-    groups[g] = make_int2((int)seg_start[lo] + off, min(ncrit, count - off));
+    const int np = min(ncrit, count - off);
+    groups[g] = make_int2((int)seg_start[lo] + off, np);
+    if (order) {
+      const bool big = 2 * np > ncrit;
+      const unsigned act = __activemask(), m = __ballot_sync(act, big), mine = big ? m : act & ~m;
+      const int leader = __ffs(mine) - 1;
+      unsigned base = 0;
+      if (lane_id() == leader) base = atomicAdd(order_count + (big ? 0 : 1), (unsigned)__popc(mine));
+      base = __shfl_sync(mine, base, leader) + (unsigned)__popc(mine & lanemask_lt());
+      const int slot = big ? (int)base : ng - 1 - (int)base;
+      if (BONSAI_IN_RANGE(slot, ng, 0x209)) order[slot] = g;
+    }
   }
 }
 
 void make_groups(const unsigned long long* sorted_ph, int n, int level_split, int ncrit, unsigned* seg_end,
                  unsigned* seg_start, unsigned* ng, unsigned* bsum, int2* groups, int group_cap, TreeInfo* info,
-                 cudaStream_t s) {
+                 int* order, unsigned* order_count, cudaStream_t s) {
   const int nbins = 1 << (3 * level_split);
   const int shift = 63 - 3 * level_split;
+  if (order) cudaMemsetAsync(order_count, 0, 2 * sizeof(unsigned), s);
   cudaMemsetAsync(seg_start, 0, sizeof(unsigned) * (size_t)nbins, s);
   cudaMemsetAsync(seg_end, 0, sizeof(unsigned) * (size_t)nbins, s);
   k_group_bounds<<<1184, 256, 0, s>>>(sorted_ph, n, shift, nbins, seg_start, seg_end);
   k_group_sizes<<<(nbins + 255) / 256, 256, 0, s>>>(seg_start, seg_end, nbins, ncrit, ng);
   exclusive_scan(ng, ng, nbins, bsum, (unsigned*)&info->ngroups, s);
-  k_group_write<<<1184, 256, 0, s>>>(seg_end, seg_start, ng, nbins, ncrit, groups, group_cap, info, n);
+  k_group_write<<<1184, 256, 0, s>>>(seg_end, seg_start, ng, nbins, ncrit, groups, group_cap, info, n, order,
+                                    order_count);
 }
 
 // Ensembles.  Bins repeat from system to system, so segments are numbered by
@@ -126,8 +143,10 @@ __global__ void __launch_bounds__(256) k_seg_group_sizes(const unsigned* __restr
 
 void make_groups_sys(const unsigned long long* sorted_ph, int n, int level_split, int ncrit, const int* sys_off,
                      int nsys, unsigned* flag, unsigned* sid, unsigned* seg_beg, unsigned* seg_end, unsigned* nseg,
-                     unsigned* bsum, int2* groups, int group_cap, TreeInfo* info, cudaStream_t s) {
+                     unsigned* bsum, int2* groups, int group_cap, TreeInfo* info, int* order, unsigned* order_count,
+                     cudaStream_t s) {
   const int shift = 63 - 3 * level_split;
+  if (order) cudaMemsetAsync(order_count, 0, 2 * sizeof(unsigned), s);
   k_seg_flags<<<1184, 256, 0, s>>>(sorted_ph, n, shift, flag);
   k_seg_mark_systems<<<(nsys + 255) / 256, 256, 0, s>>>(sys_off, nsys, flag);
   exclusive_scan(flag, sid, n, bsum, nseg, s);
@@ -135,7 +154,7 @@ void make_groups_sys(const unsigned long long* sorted_ph, int n, int level_split
   unsigned* ng = flag;
   k_seg_group_sizes<<<1184, 256, 0, s>>>(seg_beg, seg_end, nseg, n, ncrit, ng);
   exclusive_scan(ng, ng, n, bsum, (unsigned*)&info->ngroups, s);
-  k_group_write<<<1184, 256, 0, s>>>(seg_end, seg_beg, ng, n, ncrit, groups, group_cap, info, n);
+  k_group_write<<<1184, 256, 0, s>>>(seg_end, seg_beg, ng, n, ncrit, groups, group_cap, info, n, order, order_count);
 }
 
 // state gather: out[k] = in[perm[k]] for positions, velocities and ids

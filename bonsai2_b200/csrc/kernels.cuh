@@ -67,10 +67,11 @@ __global__ void k_multipoles_ref_layout(const TreeInfo* __restrict__ info, const
 // groups.cu
 void make_groups(const unsigned long long* sorted_ph, int n, int level_split, int ncrit, unsigned* count,
                  unsigned* seg_start, unsigned* ng, unsigned* bsum, int2* groups, int group_cap, TreeInfo* info,
-                 cudaStream_t s);
+                 int* order, unsigned* order_count, cudaStream_t s);
 void make_groups_sys(const unsigned long long* sorted_ph, int n, int level_split, int ncrit, const int* sys_off,
                      int nsys, unsigned* flag, unsigned* sid, unsigned* seg_beg, unsigned* seg_end, unsigned* nseg,
-                     unsigned* bsum, int2* groups, int group_cap, TreeInfo* info, cudaStream_t s);
+                     unsigned* bsum, int2* groups, int group_cap, TreeInfo* info, int* order, unsigned* order_count,
+                     cudaStream_t s);
 __global__ void k_gather_state(const int* __restrict__ perm, int n, const float4* __restrict__ pos,
                                const float4* __restrict__ vel, const int* __restrict__ id, float4* __restrict__ pos_o,
                                float4* __restrict__ vel_o, int* __restrict__ id_o);
@@ -101,7 +102,8 @@ struct PrevEval {
 };
 
 // walk.cu
-int walk_variant(int ncrit, int layout);
+constexpr int kWalkVariants = 10;
+int walk_variant(int n, int ncrit, int layout, int* parts);
 int walk_blocks_per_sm(int variant);
 // group_inv_theta == nullptr: the fixed opening angle baked into cell_open.w;
 // else 1/theta per group with (l, s) from cell_ls
@@ -110,8 +112,8 @@ void launch_walk(int variant, int nblocks, const int2* groups, const TreeInfo* i
                  const float4* cell_ls, const float* group_inv_theta, float eps2, float4* acc, int* ring_pool,
                  int ring_cap, unsigned* group_counter, unsigned long long* stats, int* status, const int* sys_off,
                  int nsys, const int* root_beg, const float4* ipos_lo, const float4* jpos_lo, const float4* cell_lo,
-                 uint2* group_counts, const int* group_list, const unsigned* group_list_n, const RelativeArgs& rel,
-                 cudaStream_t s);
+                 uint2* group_counts, const int* group_list, const unsigned* group_list_n, int parts,
+                 const RelativeArgs& rel, cudaStream_t s);
 
 // walk64.cu: the FP64 checker walk (same interaction lists as the float walk)
 void launch_walk64(int nblocks, const int2* groups, const TreeInfo* info, const float4* ipos, const float4* ipos_lo,

@@ -32,6 +32,12 @@ namespace {
 constexpr float kStartAlpha = 1e-2f;
 constexpr int kRingCap = 16384;  // per-warp level lists of the walk (ints): two halves of 8192
 constexpr int kMaxLevelSplit = 7;
+// Particles up to which the walk takes the groups more than half full first, so
+// that long ones do not run alone at its end: 250,007 particles 853 -> 725 us,
+// 2^20 2955 -> 2869; an ensemble of 1.7M 4.76 -> 4.87 ms (neighbours in the tree
+// apart, and no end to speak of).  Up to this size gcap is the particle count, so
+// the order always covers every group.
+constexpr int kOrderMax = 1 << 20;
 
 template <class T>
 cudaError_t dalloc(T** p, size_t n) {
@@ -101,9 +107,11 @@ struct Handle {
   void* mlp_wh = nullptr;
   bool mlp_loaded = false;
   int2* groups = nullptr;
+  int* group_order = nullptr;  // the order the walk takes them in (kOrderMax)
+  unsigned* order_count = nullptr;
   unsigned *g_count = nullptr, *g_seg = nullptr, *g_ng = nullptr;
   int* ring = nullptr;
-  int walk_blocks[6] = {0, 0, 0, 0, 0, 0};  // per walk variant (walk_variant)
+  int walk_blocks[kWalkVariants] = {};  // per walk variant (walk_variant)
   int ring_warps = 0;
   unsigned* group_counter = nullptr;
   unsigned long long* stats = nullptr;
@@ -248,7 +256,7 @@ struct Handle {
     dfree(&acc); dfree(&jpos); dfree(&tkey); dfree(&pkey); dfree(&kalt);
     dfree(&tperm); dfree(&pperm); dfree(&valt); dfree(&sort_counts); dfree(&bsum);
     dfree(&kalt2); dfree(&valt2); dfree(&sort_counts2);
-    dfree(&chain); dfree(&hist); dfree(&groups); dfree(&group_inv); dfree(&group_tau); dfree(&group_amag);
+    dfree(&chain); dfree(&hist); dfree(&groups); dfree(&group_order); dfree(&group_inv); dfree(&group_tau); dfree(&group_amag);
     dfree(&group_stats); dfree(&part_gid); dfree(&group_feat);
     dfree(&group_counts); dfree(&acc64); dfree(&acc64_tmp);
     release_cells();
@@ -265,7 +273,7 @@ struct Handle {
     release_particles();
     dfree(&info); dfree(&g_count); dfree(&g_seg); dfree(&g_ng); dfree(&ring);
     dfree(&group_counter); dfree(&stats); dfree(&move_partial); dfree(&energies);
-    dfree(&move_ticket); dfree(&box_ticket); dfree(&mp_barrier); dfree(&closing); dfree(&acc_valid); dfree(&box); dfree(&box_partial);
+    dfree(&move_ticket); dfree(&box_ticket); dfree(&mp_barrier); dfree(&order_count); dfree(&closing); dfree(&acc_valid); dfree(&box); dfree(&box_partial);
     dfree(&ph_table); dfree(&direct_part); dfree(&direct_out); dfree(&direct_sample);
     dfree(&mlp_w);
     if (mlp_wh) { cudaFree(mlp_wh); mlp_wh = nullptr; }
@@ -326,8 +334,8 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&g_count, (size_t)1 << (3 * kMaxLevelSplit)));
     BONSAI_CUDA_TRY(dalloc(&g_seg, (size_t)1 << (3 * kMaxLevelSplit)));
     BONSAI_CUDA_TRY(dalloc(&g_ng, (size_t)1 << (3 * kMaxLevelSplit)));
-    for (int k = 0; k < 6; k++) walk_blocks[k] = nsm * walk_blocks_per_sm(k);
-    ring_warps = *std::max_element(walk_blocks, walk_blocks + 6) * (kWalkThreads / 32);
+    for (int k = 0; k < kWalkVariants; k++) walk_blocks[k] = nsm * walk_blocks_per_sm(k);
+    ring_warps = *std::max_element(walk_blocks, walk_blocks + kWalkVariants) * (kWalkThreads / 32);
     BONSAI_CUDA_TRY(dalloc(&ring, (size_t)ring_warps * kRingCap));
     BONSAI_CUDA_TRY(dalloc(&group_counter, 1));
     BONSAI_CUDA_TRY(dalloc(&stats, 4));
@@ -337,6 +345,7 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&move_ticket, 1));
     BONSAI_CUDA_TRY(dalloc(&box_ticket, 1));
     BONSAI_CUDA_TRY(dalloc(&mp_barrier, 1));
+    BONSAI_CUDA_TRY(dalloc(&order_count, 2));
     mp_level_blocks = multipole_level_blocks(nsm);
     BONSAI_CUDA_TRY(cudaMemset(move_ticket, 0, sizeof(unsigned)));
     BONSAI_CUDA_TRY(cudaMemset(box_ticket, 0, sizeof(unsigned)));
@@ -385,6 +394,7 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&hist, tree_hist_words(nn)));
     BONSAI_CUDA_TRY(cudaMemset(hist, 0, tree_hist_words(nn) * sizeof(unsigned)));
     BONSAI_CUDA_TRY(dalloc(&groups, N));
+    if (nn <= kOrderMax) BONSAI_CUDA_TRY(dalloc(&group_order, N));
     // group-indexed arrays of the per-group angle: at most N/nCrit groups plus
     // one partial group per PH segment (groups.cu)
     gcap = (int)std::min<long long>(N, (long long)N / std::max(1, prm.ncrit) + (1ll << (3 * kMaxLevelSplit)) + 1);
@@ -507,9 +517,10 @@ struct Handle {
       // ka (8 bytes per particle) is free after the sort: segment flags and indices
       unsigned* flag = reinterpret_cast<unsigned*>(ka);
       make_groups_sys(pkey, n, ls, ncrit, sys_off, nsys, flag, flag + n, seg_beg, seg_end, nseg, bsum, groups,
-                      theta_mode ? gcap : n, info, s);
+                      theta_mode ? gcap : n, info, group_order, order_count, s);
     } else {
-      make_groups(pkey, n, ls, ncrit, g_count, g_seg, g_ng, bsum, groups, theta_mode ? gcap : n, info, s);
+      make_groups(pkey, n, ls, ncrit, g_count, g_seg, g_ng, bsum, groups, theta_mode ? gcap : n, info,
+                  group_order, order_count, s);
     }
     const int q = par ^ 1;
     k_gather_state<<<nsm * 8, 256, 0, s>>>(pperm, n, pos[par], vel[par], id[par], pos[q], vel[q], id[q]);
@@ -543,7 +554,8 @@ struct Handle {
     cudaStreamWaitEvent(st, ev_join, 0);
   }
   void enq_forces(int ncrit) {
-    const int k = walk_variant(ncrit, walk_layout);
+    int parts = 1;
+    const int k = walk_variant(n, ncrit, walk_layout, &parts);
     cudaMemsetAsync(group_counter, 0, sizeof(unsigned), st);
     cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), st);
     const float* ginv = nullptr;
@@ -576,7 +588,9 @@ struct Handle {
     launch_walk(k, walk_blocks[k], groups, info, pos[par], jpos, cell_data, cell_open, cell_stage, cell_ls,
                 ginv, prm.eps * prm.eps, acc, ring, kRingCap, group_counter, stats, &info->status, so(), nsys, root_beg,
                 precision ? plo[par] : nullptr, jlo, cell_lo, ginv ? group_counts : nullptr,
-                walk_list_on ? walk_list : nullptr, walk_list_on ? walk_list_n : nullptr, rel, st);
+                walk_list_on ? walk_list : group_order,
+                walk_list_on ? walk_list_n : (group_order ? (const unsigned*)&info->ngroups : nullptr), parts, rel,
+                st);
     acc_in_state_order = true;
   }
   void enq_move(bool write) {

@@ -57,9 +57,6 @@ constexpr int kWalkWarps = kWalkThreads / 32;
 #define BONSAI_DO_PRAGMA(x) _Pragma(#x)
 #define BONSAI_UNROLL_N(n) BONSAI_DO_PRAGMA(unroll n)
 
-#ifndef BONSAI_WALK_PACKED
-#define BONSAI_WALK_PACKED 1
-#endif
 // children of opened nodes written by their parent's lane (1) or expanded
 // 32 at a time by a shuffle search over the warp's scan (0)
 #ifndef BONSAI_WALK_CHILD_LOOP
@@ -97,6 +94,11 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   *static_cast<float4*>(smem) = __ldg(static_cast<const float4*>(gmem));
 #endif
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // direct-source ring per warp (a power of two, >= 64)
@@ -115,8 +117,9 @@ constexpr int kDirRing = 128;
 // sm_100: one instruction per pair, same FP32 pipe rate, half the issue
 // slots).  Sources are scalars broadcast into both halves.
 __device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ float vmul(float a, float b) { return a * b; }
-__device__ __forceinline__ float vadd(float a, float b) { return a + b; }
+// (not contracted, so that both forms round alike)
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float vrsqrt(float a) { return rsqrtf(a); }
 __device__ __forceinline__ float vdup(float a, float) { return a; }
 __device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
@@ -178,16 +181,12 @@ __device__ __forceinline__ void mono_acc(AVec<V>& acc, const IVec<V>& p, const f
   acc.z = vfma(mr3, dz, acc.z);
 }
 
-// NI i-particles of a lane as NV vectors of type V
+// NI i-particles of a lane as NV vectors of type V: rows 2v and 2v + 1 in
+// vector v, or one row in a scalar
 template <int NI>
 struct Lanes {
-#if BONSAI_WALK_PACKED
   typedef typename std::conditional<(NI >= 2), float2, float>::type V;
   static constexpr int NV = NI >= 2 ? NI / 2 : NI;
-#else
-  typedef float V;
-  static constexpr int NV = NI;
-#endif
 };
 
 __device__ __forceinline__ void set_lane(float& v, int, float x) { v = x; }
@@ -197,11 +196,54 @@ __device__ __forceinline__ void set_lane(float2& v, int h, float x) {
 __device__ __forceinline__ float get_lane(float v, int) { return v; }
 __device__ __forceinline__ float get_lane(float2 v, int h) { return h ? v.y : v.x; }
 
-// Particle ownership.  SPLIT: lane l holds particles (l & 15) + 16k, k < NI,
-// both half-warps hold the same particles, the two halves evaluate alternate
-// entries of every 32-entry batch and their sums are added once per group, so
-// each broadcast shared-memory load feeds NI (= 4 for nCrit <= 64)
-// interactions.  Otherwise lane l holds l + 32k, k < NI.
+// a vector's first row on its own (groups of one row)
+__device__ __forceinline__ IVec<float> first_row(const IVec<float>& v) { return v; }
+__device__ __forceinline__ IVec<float> first_row(const IVec<float2>& v) { return {v.nx.x, v.ny.x, v.nz.x}; }
+__device__ __forceinline__ AVec<float> first_row(const AVec<float>& v) { return v; }
+__device__ __forceinline__ AVec<float> first_row(const AVec<float2>& v) { return {v.x.x, v.y.x, v.z.x, v.w.x}; }
+__device__ __forceinline__ void put_first_row(AVec<float>& v, const AVec<float>& r) { v = r; }
+__device__ __forceinline__ void put_first_row(AVec<float2>& v, const AVec<float>& r) {
+  v.x.x = r.x; v.y.x = r.y; v.z.x = r.z; v.w.x = r.w;
+}
+
+// Sources A[0], A[js], .. below count for a lane's NV vectors (JS: the
+// compile-time stride), or for its first row alone
+template <int JS, int NV, class V>
+__device__ __forceinline__ void quad_batch(AVec<V>* av, const IVec<V>* iv, const float4* A0, const float4* A1,
+                                           const float4* A2, V eps2) {
+  BONSAI_UNROLL_N(BONSAI_WALK_UNROLL)
+  for (int j = 0; j < 32; j += JS) {
+    const float4 a0 = A0[j], a1 = A1[j], a2 = A2[j];
+#pragma unroll
+    for (int v = 0; v < NV; v++) quad_acc(av[v], iv[v], a0, a1, a2, eps2);
+  }
+}
+template <int JS, int NV, class V>
+__device__ __forceinline__ void mono_batch(AVec<V>* av, const IVec<V>* iv, const float4* D, V eps2) {
+  BONSAI_UNROLL_N(BONSAI_WALK_UNROLL)
+  for (int j = 0; j < 32; j += JS) {
+    const float4 pj = D[j];
+#pragma unroll
+    for (int v = 0; v < NV; v++) mono_acc(av[v], iv[v], pj, eps2);
+  }
+}
+
+// Particle ownership.  A row is STRIDE particles, one per lane: 16 with SPLIT,
+// where both half-warps hold the same rows, evaluate alternate entries of every
+// 32-entry batch and are added once per group, so that each broadcast
+// shared-memory load feeds NI (= 4 for nCrit <= 64) interactions; else 32.
+// Lane l holds particles (l % STRIDE) + STRIDE k of the group, k < NI.
+// A group's empty rows are not evaluated: the batches run on the vectors that
+// hold particles, and a group of one row in scalar arithmetic; with at most 16
+// particles the lanes beyond the next power of two take sources instead (8
+// lanes per row: 4 streams of sources, and so on), added by shuffles at the
+// end.  (PH segments end in partly filled groups: at nCrit 64 a Plummer sphere
+// of 2^18 has 31 particles per group, a galaxy of 10^5 12, one of 2^24 63.)
+// SHARE (few groups): `parts` warps share a group, each walking the whole list
+// for its own NI rows (part p those from p NI on; a part past the last particle
+// does nothing).  The box is that of the whole group, so every part takes the
+// same decisions; a particle's sources, their order and the streams they fall
+// into depend on the group alone, so the forces do not depend on parts.
 // PERGROUP: each group has its own opening angle (1/theta_g in
 // group_inv_theta); the opening size is re-formed as (l/theta_g + s)^2 from
 // cell_ls with the same rounding as the multipole kernel, so theta_g = theta
@@ -215,7 +257,7 @@ __device__ __forceinline__ float get_lane(float2 v, int h) { return h ? v.y : v.
 // position) as (hi - R) + lo: the subtraction is exact for nearby points, so
 // separations keep FP32 relative precision however far from the origin the
 // group lies.  The interaction loops are unchanged.
-template <int NI, bool SPLIT, bool PERGROUP, bool ENS, bool DS>
+template <int NI, bool SPLIT, bool PERGROUP, bool ENS, bool DS, bool SHARE>
 __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
     k_walk(const int2* __restrict__ groups, const TreeInfo* __restrict__ info, const float4* __restrict__ ipos,
            const float4* __restrict__ jpos, const uint4* __restrict__ cell_data,
@@ -227,7 +269,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
            int nsys, const int* __restrict__ root_beg, const float4* __restrict__ ipos_lo,
            const float4* __restrict__ jpos_lo, const float4* __restrict__ cell_lo,
            uint2* __restrict__ group_counts, const int* __restrict__ group_list,
-           const unsigned* __restrict__ group_list_n, const RelativeArgs rel) {
+           const unsigned* __restrict__ group_list_n, int parts, const RelativeArgs rel) {
   constexpr int STRIDE = SPLIT ? 16 : 32;
   constexpr int JSTEP = SPLIT ? 2 : 1;
   __shared__ float4 s_a0[kWalkWarps][64];
@@ -238,8 +280,6 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
   __shared__ float4 s_d[kWalkWarps][DRING];
   __shared__ float4 s_dlo[kWalkWarps][DSA ? DRING : 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int sub = SPLIT ? (lane & 15) : lane;
-  const int half = SPLIT ? (lane >> 4) : 0;
   // two halves of the warp's list buffer: the current level is read from one
   // while the next is written to the other, so the hot footprint stays ~2x the
   // widest level (a sweeping ring would push its dirty lines out to HBM)
@@ -258,16 +298,29 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
   bool start_fallback = false;
   if (rel.acc_valid && blockIdx.x == 0 && threadIdx.x == 0) start_fallback = rel.acc_valid[0] == 0;
 
-  while (true) {
-    int g = 0;
-    if (lane == 0) g = (int)atomicAdd(group_counter, 1u);
-    g = __shfl_sync(kFull, g, 0);
+  // SHARE: the first unit of each warp is fixed, the warps of a block far apart,
+  // so that few units still spread over all SMs; the others come from the counter
+  [[maybe_unused]] int unit = w * (int)gridDim.x + (int)blockIdx.x;
+  for (bool first = SHARE;; first = false) {
+    int g = 0, row0 = 0;
+    if (SHARE) {
+      if (!first) {
+        if (lane == 0) unit = (int)(gridDim.x * kWalkWarps + atomicAdd(group_counter, 1u));
+        unit = __shfl_sync(kFull, unit, 0);
+      }
+      g = unit / parts;
+      row0 = (unit - g * parts) * NI;
+    } else {
+      if (lane == 0) g = (int)atomicAdd(group_counter, 1u);
+      g = __shfl_sync(kFull, g, 0);
+    }
     if (g >= ngroups) break;
     if (group_list) g = __ldg(group_list + g);
     if (!BONSAI_IN_RANGE(g, ngroups_all, 0x401)) continue;
     const int2 gd = groups[g];
     const int pbeg = gd.x, np = gd.y;
-    if (!BONSAI_IN_RANGE(np - 1, NI * STRIDE, 0x402) || !BONSAI_IN_RANGE(pbeg + np - 1, npart, 0x403) ||
+    if (SHARE && row0 * STRIDE >= np) continue;
+    if (!BONSAI_IN_RANGE(np - 1, NI * STRIDE * (SHARE ? parts : 1), 0x402) || !BONSAI_IN_RANGE(pbeg + np - 1, npart, 0x403) ||
         !BONSAI_IN_RANGE(pbeg, npart, 0x407))
       continue;
     const float inv_theta_g = PERGROUP ? group_inv_theta[g] : 0.0f;
@@ -285,6 +338,11 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
     }
     typedef typename Lanes<NI>::V V;
     constexpr int NV = Lanes<NI>::NV;
+    // rows with particles; lanes per row and the stream of sources of this lane
+    const int rows = (np + STRIDE - 1) / STRIDE - row0;
+    const int lp = np > 16 ? STRIDE : (np > 1 ? 1 << (32 - __clz(np - 1)) : 1);
+    const int sub = lane & (lp - 1);
+    const int js = 32 / lp, stream = lane / lp;
     IPart pi[NI];
     float3 R = make_float3(0.f, 0.f, 0.f);
     if (DS) {
@@ -292,21 +350,25 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
       R = make_float3(r0.x, r0.y, r0.z);
     }
     float mnx = 3.0e38f, mny = 3.0e38f, mnz = 3.0e38f, mxx = -3.0e38f, mxy = -3.0e38f, mxz = -3.0e38f;
-#pragma unroll
-    for (int k = 0; k < NI; k++) {
-      const int ii = pbeg + min(k * STRIDE + sub, np - 1);
+    auto load_row = [&](int row) {
+      const int ii = pbeg + min(row * STRIDE + sub, np - 1);
       const float4 p = ipos[ii];
+      IPart q = {p.x, p.y, p.z};
       if (DS) {
         const float4 lo = ipos_lo[ii];
-        pi[k].x = __fadd_rn(__fsub_rn(p.x, R.x), lo.x);
-        pi[k].y = __fadd_rn(__fsub_rn(p.y, R.y), lo.y);
-        pi[k].z = __fadd_rn(__fsub_rn(p.z, R.z), lo.z);
-      } else {
-        pi[k].x = p.x; pi[k].y = p.y; pi[k].z = p.z;
+        q.x = __fadd_rn(__fsub_rn(p.x, R.x), lo.x);
+        q.y = __fadd_rn(__fsub_rn(p.y, R.y), lo.y);
+        q.z = __fadd_rn(__fsub_rn(p.z, R.z), lo.z);
       }
-      mnx = fminf(mnx, pi[k].x); mny = fminf(mny, pi[k].y); mnz = fminf(mnz, pi[k].z);
-      mxx = fmaxf(mxx, pi[k].x); mxy = fmaxf(mxy, pi[k].y); mxz = fmaxf(mxz, pi[k].z);
-    }
+      mnx = fminf(mnx, q.x); mny = fminf(mny, q.y); mnz = fminf(mnz, q.z);
+      mxx = fmaxf(mxx, q.x); mxy = fmaxf(mxy, q.y); mxz = fmaxf(mxz, q.z);
+      return q;
+    };
+#pragma unroll
+    for (int k = 0; k < NI; k++) pi[k] = load_row(row0 + k);
+    if (SHARE)  // the other parts' rows, for the box
+      for (int row = 0; row * STRIDE < np; row++)
+        if (row < row0 || row >= row0 + NI) load_row(row);
     mnx = warp_min_f32(mnx); mny = warp_min_f32(mny); mnz = warp_min_f32(mnz);
     mxx = warp_max_f32(mxx); mxy = warp_max_f32(mxy); mxz = warp_max_f32(mxz);
     const float3 gc = make_float3(__fmul_rn(0.5f, __fadd_rn(mxx, mnx)), __fmul_rn(0.5f, __fadd_rn(mxy, mny)),
@@ -318,9 +380,9 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
     AVec<V> av[NV];
 #pragma unroll
     for (int k = 0; k < NI; k++) {
-      set_lane(iv[k % NV].nx, k / NV, -pi[k].x);
-      set_lane(iv[k % NV].ny, k / NV, -pi[k].y);
-      set_lane(iv[k % NV].nz, k / NV, -pi[k].z);
+      set_lane(iv[k / 2].nx, k & 1, -pi[k].x);
+      set_lane(iv[k / 2].ny, k & 1, -pi[k].y);
+      set_lane(iv[k / 2].nz, k & 1, -pi[k].z);
     }
 #pragma unroll
     for (int v = 0; v < NV; v++) av[v].x = av[v].y = av[v].z = av[v].w = vdup(0.0f, V());
@@ -336,14 +398,19 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
     // evaluation of the staged 32-entry batches (ring order): the accepted
     // cells' quadrupoles and the opened leaves' particles
     auto eval_app = [&]() {
-      const float4* A0 = &s_a0[w][a_head + half];
-      const float4* A1 = &s_a1[w][a_head + half];
-      const float4* A2 = &s_a2[w][a_head + half];
-      BONSAI_UNROLL_N(BONSAI_WALK_UNROLL)
-      for (int j = 0; j < 32; j += JSTEP) {
-        const float4 a0 = A0[j], a1 = A1[j], a2 = A2[j];
-#pragma unroll
-        for (int v = 0; v < NV; v++) quad_acc(av[v], iv[v], a0, a1, a2, veps2);
+      const float4* A0 = &s_a0[w][a_head + stream];
+      const float4* A1 = &s_a1[w][a_head + stream];
+      const float4* A2 = &s_a2[w][a_head + stream];
+      if (NI > 2 && rows > 2) {
+        quad_batch<JSTEP, NV>(av, iv, A0, A1, A2, veps2);
+      } else if (NI > 1 && rows > 1) {
+        quad_batch<JSTEP, 1>(av, iv, A0, A1, A2, veps2);
+      } else {
+        AVec<float> r = first_row(av[0]);
+        const IVec<float> p = first_row(iv[0]);
+        BONSAI_UNROLL_N(BONSAI_WALK_UNROLL)
+        for (int j = 0; j < 32; j += js) quad_acc(r, p, A0[j], A1[j], A2[j], eps2);
+        put_first_row(av[0], r);
       }
       a_head = (a_head + 32) & 63;
       a_cnt -= 32;
@@ -365,12 +432,17 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
     };
     auto eval_dir = [&]() {
       if (DSA) combine_dir(0, 32);
-      const float4* D = &s_d[w][d_head + half];
-      BONSAI_UNROLL_N(BONSAI_WALK_UNROLL)
-      for (int j = 0; j < 32; j += JSTEP) {
-        const float4 pj = D[j];
-#pragma unroll
-        for (int v = 0; v < NV; v++) mono_acc(av[v], iv[v], pj, veps2);
+      const float4* D = &s_d[w][d_head + stream];
+      if (NI > 2 && rows > 2) {
+        mono_batch<JSTEP, NV>(av, iv, D, veps2);
+      } else if (NI > 1 && rows > 1) {
+        mono_batch<JSTEP, 1>(av, iv, D, veps2);
+      } else {
+        AVec<float> r = first_row(av[0]);
+        const IVec<float> p = first_row(iv[0]);
+        BONSAI_UNROLL_N(BONSAI_WALK_UNROLL)
+        for (int j = 0; j < 32; j += js) mono_acc(r, p, D[j], eps2);
+        put_first_row(av[0], r);
       }
       d_head = (d_head + 32) & (DRING - 1);
       d_cnt -= 32;
@@ -519,8 +591,11 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
           const int f = __shfl_sync(kFull, pb, src);
           const int e = __shfl_sync(kFull, incl2 - nb, src);
           const int cnt = min(32, tot2 - base);
-          if (d_cnt + cnt > DRING) {  // no room: evaluate one batch now
-            cp_async_wait_all();
+          if (d_cnt + cnt > DRING) {
+            // no room: evaluate the oldest batch now.  Each step of this loop is
+            // one group of copies of at most 32 particles, so with the 128-entry
+            // ring the batch is older than the two last groups, which stay in flight
+            cp_async_wait_group<DRING == 128 ? 2 : 0>();
             __syncwarp();
             eval_dir();
             __syncwarp();
@@ -543,6 +618,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
               cp_async16(dst, jpos + jj);
             }
           }
+          cp_async_commit();
           d_cnt += cnt;
         }
       }
@@ -555,7 +631,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
     // the remaining batches, full and partial
     cp_async_wait_all();
     __syncwarp();
-    for (int j = half; j < a_cnt; j += JSTEP) {
+    for (int j = stream; j < a_cnt; j += js) {
       const int sl = (a_head + j) & 63;
       const float4 a0 = s_a0[w][sl], a1 = s_a1[w][sl], a2 = s_a2[w][sl];
 #pragma unroll
@@ -563,7 +639,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
     }
     n_app += a_cnt;
     if (DSA) combine_dir(0, d_cnt);
-    for (int j = half; j < d_cnt; j += JSTEP) {
+    for (int j = stream; j < d_cnt; j += js) {
       const float4 pj = s_d[w][(d_head + j) & (DRING - 1)];
 #pragma unroll
       for (int v = 0; v < NV; v++) mono_acc(av[v], iv[v], pj, veps2);
@@ -573,8 +649,9 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
     float4 ai[NI];
 #pragma unroll
     for (int k = 0; k < NI; k++)
-      ai[k] = make_float4(get_lane(av[k % NV].x, k / NV), get_lane(av[k % NV].y, k / NV),
-                          get_lane(av[k % NV].z, k / NV), -get_lane(av[k % NV].w, k / NV));
+      ai[k] = make_float4(get_lane(av[k / 2].x, k & 1), get_lane(av[k / 2].y, k & 1),
+                          get_lane(av[k / 2].z, k & 1), -get_lane(av[k / 2].w, k & 1));
+    // the streams' sums
     if (SPLIT) {
 #pragma unroll
       for (int k = 0; k < NI; k++) {
@@ -584,19 +661,26 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
         ai[k].w += __shfl_xor_sync(kFull, ai[k].w, 16);
       }
     }
+    for (int o = SPLIT ? 8 : 16; o >= lp; o >>= 1) {
+      ai[0].x += __shfl_xor_sync(kFull, ai[0].x, o);
+      ai[0].y += __shfl_xor_sync(kFull, ai[0].y, o);
+      ai[0].z += __shfl_xor_sync(kFull, ai[0].z, o);
+      ai[0].w += __shfl_xor_sync(kFull, ai[0].w, o);
+    }
 
     if (overflow) {
       if (lane == 0) set_status(status, kStatusWalkStack);
 #pragma unroll
       for (int k = 0; k < NI; k++) ai[k] = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
     }
-    if (half == 0) {
+    if (stream == 0) {
 #pragma unroll
       for (int k = 0; k < NI; k++) {
-        const int idx = k * STRIDE + sub;
+        const int idx = (row0 + k) * STRIDE + sub;
         if (idx < np) acc[pbeg + idx] = ai[k];
       }
     }
+    if (SHARE && row0) continue;  // counts and statistics: once per group
     // per-group (approximate, direct) interaction counts, for the per-group angle variant
     if (PERGROUP && group_counts && lane == 0) group_counts[g] = make_uint2(n_app, n_dir);
     if (PERGROUP && rel.stats) {
@@ -631,13 +715,28 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
 }
 
 // variants: 0..2 half-warp split with NI = 1, 2, 4 (nCrit <= 16, 32, 64);
-// 3..5 full warp with NI = 1, 2, 4 (nCrit <= 32, 64, 128).  layout 0: split
-// where nCrit <= 64 (the default); 1: full warp.
-int walk_variant(int ncrit, int layout) {
-#if BONSAI_WALK_SPLIT
-  if (ncrit <= 64 && layout != 1) return ncrit <= 16 ? 0 : (ncrit <= 32 ? 1 : 2);
-#endif
-  return ncrit <= 32 ? 3 : (ncrit <= 64 ? 4 : 5);
+// 3..5 full warp with NI = 1, 2, 4 (nCrit <= 32, 64, 128); layout 0: split
+// where nCrit <= 64 (the default); 1: full warp.  6..9: NI = 1, 2 of each with
+// a group shared by two warps, for particles too few to fill the device with
+// groups (2368 warps): the walk then takes as long as its longest group, and
+// halving the rows of a warp outweighs walking the list twice.  The lines, by
+// measurement on a B200 (walk of the whole and the shared form, us):
+//   split, nCrit 64 (NI 4): 16,384 Plummer 342/162, 65,536 424/270, 100,000
+//     448/375, 131,072 461/479, 180,000 galaxy 721/711
+//   split, nCrit 32 (NI 2): 16,384 184/133, 40,000 field 160/178
+//   full, nCrit 128 (NI 4): 65,536 971/428, 250,007 galaxy 1463/1102, 500,000
+//     1778/1776 (galaxy 2223/1983), 2^20 3494/3650
+// and as many for the full-warp NI 2, by the particles of its rows, as for the
+// split one.  (Four warps per group were no better than two up to 16,384 and
+// worse above.)
+int walk_variant(int n, int ncrit, int layout, int* parts) {
+  const bool split = BONSAI_WALK_SPLIT && ncrit <= 64 && layout != 1;
+  const int rows = (ncrit + (split ? 15 : 31)) / (split ? 16 : 32);
+  const int v = rows <= 1 ? 0 : (rows <= 2 ? 1 : 2);
+  const int line = v == 2 ? (split ? 7 << 14 : 1 << 19) : (v == 1 ? (split ? 3 << 13 : 3 << 14) : 0);
+  const bool share = n <= line;
+  *parts = share ? 2 : 1;
+  return share ? 6 + (split ? 0 : 2) + (v - 1) : (split ? 0 : 3) + v;
 }
 
 template <class K>
@@ -649,29 +748,31 @@ static int occupancy(K kernel) {
 
 // blocks per SM that every instantiation of the variant reaches (the level
 // lists are sized for the largest grid)
-template <int NI, bool SPLIT>
+template <int NI, bool SPLIT, bool SHARE>
 static int occupancy_of() {
-  int nb = occupancy(k_walk<NI, SPLIT, false, false, false>);
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, false, false>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, true, false>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, true, false>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, true, true>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, true, true>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, false, true>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, false, true>));
+  int nb = occupancy(k_walk<NI, SPLIT, false, false, false, SHARE>);
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, false, false, SHARE>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, true, false, SHARE>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, true, false, SHARE>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, true, true, SHARE>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, true, true, SHARE>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, false, true, SHARE>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, false, true, SHARE>));
   return nb < 1 ? 1 : nb;
 }
 
 int walk_blocks_per_sm(int variant) {
   switch (variant) {
-#if BONSAI_WALK_SPLIT
-    case 0: return occupancy_of<1, true>();
-    case 1: return occupancy_of<2, true>();
-    case 2: return occupancy_of<4, true>();
-#endif
-    case 3: return occupancy_of<1, false>();
-    case 4: return occupancy_of<2, false>();
-    default: return occupancy_of<4, false>();
+    case 0: return occupancy_of<1, true, false>();
+    case 1: return occupancy_of<2, true, false>();
+    case 2: return occupancy_of<4, true, false>();
+    case 3: return occupancy_of<1, false, false>();
+    case 4: return occupancy_of<2, false, false>();
+    case 5: return occupancy_of<4, false, false>();
+    case 6: return occupancy_of<1, true, true>();
+    case 7: return occupancy_of<2, true, true>();
+    case 8: return occupancy_of<1, false, true>();
+    default: return occupancy_of<2, false, true>();
   }
 }
 
@@ -681,39 +782,41 @@ void launch_walk(int variant, int nblocks, const int2* groups, const TreeInfo* i
                  float4* acc, int* ring_pool, int ring_cap, unsigned* group_counter, unsigned long long* stats,
                  int* status, const int* sys_off, int nsys, const int* root_beg, const float4* ipos_lo,
                  const float4* jpos_lo, const float4* cell_lo, uint2* group_counts, const int* group_list,
-                 const unsigned* group_list_n, const RelativeArgs& rel, cudaStream_t s) {
+                 const unsigned* group_list_n, int parts, const RelativeArgs& rel, cudaStream_t s) {
 #define BONSAI_WALK_ARGS                                                                                          \
   groups, info, ipos, jpos, cell_data, cell_open, cell_stage, cell_ls, group_inv_theta, eps2, acc, ring_pool, \
       ring_cap, group_counter, stats, status, sys_off, nsys, root_beg, ipos_lo, jpos_lo, cell_lo, group_counts,  \
-      group_list, group_list_n, rel
-#define BONSAI_WALK(NI, SP)                                                                \
-  do {                                                                                     \
-    if (nsys > 1 && ipos_lo && group_inv_theta)                                            \
-      k_walk<NI, SP, true, true, true><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS);   \
-    else if (nsys > 1 && ipos_lo)                                                          \
-      k_walk<NI, SP, false, true, true><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS);  \
-    else if (nsys > 1 && group_inv_theta)                                                  \
-      k_walk<NI, SP, true, true, false><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS);  \
-    else if (nsys > 1)                                                                     \
-      k_walk<NI, SP, false, true, false><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS); \
-    else if (ipos_lo && group_inv_theta)                                                   \
-      k_walk<NI, SP, true, false, true><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS);  \
-    else if (ipos_lo)                                                                      \
-      k_walk<NI, SP, false, false, true><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS); \
-    else if (group_inv_theta)                                                              \
-      k_walk<NI, SP, true, false, false><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS); \
-    else                                                                                   \
-      k_walk<NI, SP, false, false, false><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS); \
+      group_list, group_list_n, parts, rel
+#define BONSAI_WALK(NI, SP, SH)                                                                \
+  do {                                                                                         \
+    if (nsys > 1 && ipos_lo && group_inv_theta)                                                \
+      k_walk<NI, SP, true, true, true, SH><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS);   \
+    else if (nsys > 1 && ipos_lo)                                                              \
+      k_walk<NI, SP, false, true, true, SH><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS);  \
+    else if (nsys > 1 && group_inv_theta)                                                      \
+      k_walk<NI, SP, true, true, false, SH><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS);  \
+    else if (nsys > 1)                                                                         \
+      k_walk<NI, SP, false, true, false, SH><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS); \
+    else if (ipos_lo && group_inv_theta)                                                       \
+      k_walk<NI, SP, true, false, true, SH><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS);  \
+    else if (ipos_lo)                                                                          \
+      k_walk<NI, SP, false, false, true, SH><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS); \
+    else if (group_inv_theta)                                                                  \
+      k_walk<NI, SP, true, false, false, SH><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS); \
+    else                                                                                       \
+      k_walk<NI, SP, false, false, false, SH><<<nblocks, kWalkThreads, 0, s>>>(BONSAI_WALK_ARGS); \
   } while (0)
   switch (variant) {
-#if BONSAI_WALK_SPLIT
-    case 0: BONSAI_WALK(1, true); break;
-    case 1: BONSAI_WALK(2, true); break;
-    case 2: BONSAI_WALK(4, true); break;
-#endif
-    case 3: BONSAI_WALK(1, false); break;
-    case 4: BONSAI_WALK(2, false); break;
-    default: BONSAI_WALK(4, false); break;
+    case 0: BONSAI_WALK(1, true, false); break;
+    case 1: BONSAI_WALK(2, true, false); break;
+    case 2: BONSAI_WALK(4, true, false); break;
+    case 3: BONSAI_WALK(1, false, false); break;
+    case 4: BONSAI_WALK(2, false, false); break;
+    case 5: BONSAI_WALK(4, false, false); break;
+    case 6: BONSAI_WALK(1, true, true); break;
+    case 7: BONSAI_WALK(2, true, true); break;
+    case 8: BONSAI_WALK(1, false, true); break;
+    default: BONSAI_WALK(2, false, true); break;
   }
 #undef BONSAI_WALK
 #undef BONSAI_WALK_ARGS
