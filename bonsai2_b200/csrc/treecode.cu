@@ -493,9 +493,10 @@ struct Handle {
       launch_sys_keys(pos[par], chunks, nchunks, chunk_beg, nsys, sys_box_part, sys_box, ph_table, tkey, pkey,
                       &info->status, nsm * 8, st);
     } else {
-      cudaMemsetAsync(box_ticket, 0, sizeof(unsigned), st);
-      k_box<<<box_blocks, 256, 0, st>>>(pos[par], n, box_partial, box_ticket, box, &info->status);
-      k_keys<<<nsm * 8, 256, 0, st>>>(pos[par], n, box, ph_table, tkey, pkey);
+      // few blocks for few particles: the last one folds a row per block
+      k_box<<<std::min(box_blocks, (n + 1023) / 1024), 256, 0, st>>>(pos[par], n, box_partial, box_ticket, box,
+                                                                     &info->status);
+      k_keys<<<std::min(nsm * 8, (n + 255) / 256), 256, 0, st>>>(pos[par], n, box, ph_table, tkey, pkey);
     }
   }
   void enq_tree(int nleaf) {
