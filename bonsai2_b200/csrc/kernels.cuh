@@ -158,7 +158,12 @@ void launch_direct_fp64(const float4* pos, int n, const int* sample, int ns, dou
                         double* part, int nsplit, double* out, cudaStream_t s, const float4* lo = nullptr);
 __global__ void k_scatter_by_id(const int* __restrict__ id, int n, const float4* __restrict__ in,
                                 float4* __restrict__ out);
-__global__ void k_iota(int* __restrict__ a, int n);
+void launch_load_state(const float4* pos, const float4* vel, int n, float4* pos_o, float4* vel_o, int* id, float4* lo,
+                       int* closing, int* acc_valid, int nblocks, cudaStream_t s);
+void launch_invert(const int* id, int n, int* inv, int nblocks, cudaStream_t s);
+// arrays in state order to the caller's order through inv (launch_invert); any dst may be null
+void launch_fetch(const int* inv, int n, const float4* const src[3], float4* const dst[3], int nblocks,
+                  cudaStream_t s);
 double fma_probe_tflops(int nsm, cudaStream_t st, float* scratch);
 int kernel_binary_version(int* binary_version, int* ptx_version);
 

@@ -895,6 +895,32 @@ int bonsai_set_params(bonsai_handle hh, const bonsai_params* p) {
   return 0;
 }
 
+// Whether a kernel on device dev may read or write `bytes` at p as float4: a
+// 16-byte aligned range inside one allocation of that device.  Anything else a
+// copy takes (another device's memory, an odd address) goes through a copy, and
+// what a copy refuses stays refused.
+static bool kernel_range(const void* p, size_t bytes, int dev) {
+  if (reinterpret_cast<uintptr_t>(p) & 15u) return false;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != dev) return false;
+  typedef int (*RangeFn)(unsigned long long*, size_t*, unsigned long long);
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+      found != cudaDriverEntryPointSuccess || !fn) {
+    cudaGetLastError();
+    return false;
+  }
+  unsigned long long base = 0;
+  size_t size = 0;
+  const unsigned long long q = reinterpret_cast<unsigned long long>(p);
+  return reinterpret_cast<RangeFn>(fn)(&base, &size, q) == 0 && q >= base && q + bytes <= base + size;
+}
+
 static int set_particles_impl(Handle* h, const float* pos4, const float* vel4, int n, cudaMemcpyKind kind) {
   if (!h) return BONSAI_ERR_HANDLE;
   if (!pos4 || !vel4 || n < 1) return BONSAI_ERR_ARG;
@@ -904,12 +930,17 @@ static int set_particles_impl(Handle* h, const float* pos4, const float* vel4, i
     if (rc) return rc;
   }
   const size_t bytes = (size_t)n * sizeof(float4);
-  BONSAI_CUDA_TRY(cudaMemcpyAsync(h->pos[h->par], pos4, bytes, kind, h->st));
-  BONSAI_CUDA_TRY(cudaMemcpyAsync(h->vel[h->par], vel4, bytes, kind, h->st));
-  k_iota<<<h->nsm * 4, 256, 0, h->st>>>(h->id[h->par], n);
-  if (h->precision) BONSAI_CUDA_TRY(cudaMemsetAsync(h->plo[h->par], 0, bytes, h->st));  // float input: lo = 0
-  BONSAI_CUDA_TRY(cudaMemsetAsync(h->closing, 0, sizeof(int), h->st));
-  BONSAI_CUDA_TRY(cudaMemsetAsync(h->acc_valid, 0, 2 * sizeof(int), h->st));  // no previous accelerations
+  const bool direct = kind == cudaMemcpyDeviceToDevice && kernel_range(pos4, bytes, h->dev) &&
+                      kernel_range(vel4, bytes, h->dev);
+  if (!direct) {
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(h->pos[h->par], pos4, bytes, kind, h->st));
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(h->vel[h->par], vel4, bytes, kind, h->st));
+  }
+  // float input: the low parts of double-single positions are 0
+  launch_load_state(direct ? reinterpret_cast<const float4*>(pos4) : nullptr,
+                    direct ? reinterpret_cast<const float4*>(vel4) : nullptr, n, h->pos[h->par], h->vel[h->par],
+                    h->id[h->par], h->precision ? h->plo[h->par] : nullptr, h->closing, h->acc_valid, h->nsm * 8,
+                    h->st);
   h->built = h->mp_done = h->grouped = h->forced = h->moved_after_forces = false;
   h->bts_ready = false;
   return last_cuda();
@@ -928,13 +959,30 @@ static int get_particles_impl(Handle* h, float* pos4, float* vel4, float* acc4, 
   BONSAI_CUDA_TRY(cudaSetDevice(h->dev));
   const int n = h->n;
   const size_t bytes = (size_t)n * sizeof(float4);
-  float4* tmp = h->pos[h->par ^ 1];  // the idle state buffer
   const float4* src[3] = {h->pos[h->par], h->vel[h->par], h->acc};
   float* dst[3] = {pos4, vel4, acc4};
-  for (int k = 0; k < 3; k++) {
-    if (!dst[k]) continue;
-    k_scatter_by_id<<<h->nsm * 8, 256, 0, h->st>>>(h->id[h->par], n, src[k], tmp);
-    BONSAI_CUDA_TRY(cudaMemcpyAsync(dst[k], tmp, bytes, kind, h->st));
+  if (!pos4 && !vel4 && !acc4) {
+    BONSAI_CUDA_TRY(cudaStreamSynchronize(h->st));
+    return last_cuda();
+  }
+  int* inv = h->valt;  // the sort's scratch, idle between builds
+  launch_invert(h->id[h->par], n, inv, h->nsm * 8, h->st);
+  float4* out[3] = {nullptr, nullptr, nullptr};
+  bool direct = kind == cudaMemcpyDeviceToDevice;
+  for (int k = 0; k < 3; k++) direct = direct && (!dst[k] || kernel_range(dst[k], bytes, h->dev));
+  if (direct) {
+    for (int k = 0; k < 3; k++) out[k] = reinterpret_cast<float4*>(dst[k]);
+    launch_fetch(inv, n, src, out, h->nsm * 8, h->st);
+  } else {
+    // through the two idle state buffers in turn
+    for (int k = 0; k < 3; k++) {
+      if (!dst[k]) continue;
+      float4* tmp = k == 1 ? h->vel[h->par ^ 1] : h->pos[h->par ^ 1];
+      float4* one[3] = {tmp, nullptr, nullptr};
+      const float4* from[3] = {src[k], nullptr, nullptr};
+      launch_fetch(inv, n, from, one, h->nsm * 8, h->st);
+      BONSAI_CUDA_TRY(cudaMemcpyAsync(dst[k], tmp, bytes, kind, h->st));
+    }
   }
   BONSAI_CUDA_TRY(cudaStreamSynchronize(h->st));
   return last_cuda();
@@ -966,13 +1014,9 @@ int bonsai_set_particles_async(bonsai_handle hh, const float* pos4, const float*
   BONSAI_CUDA_TRY(cudaEventRecord(h->ev_in_copied, h->st_h2d));
   // the handle's stream takes the particles over when they have landed
   BONSAI_CUDA_TRY(cudaStreamWaitEvent(h->st, h->ev_in_copied, 0));
-  BONSAI_CUDA_TRY(cudaMemcpyAsync(h->pos[h->par], h->in_pos, bytes, cudaMemcpyDeviceToDevice, h->st));
-  BONSAI_CUDA_TRY(cudaMemcpyAsync(h->vel[h->par], h->in_vel, bytes, cudaMemcpyDeviceToDevice, h->st));
+  launch_load_state(h->in_pos, h->in_vel, n, h->pos[h->par], h->vel[h->par], h->id[h->par],
+                    h->precision ? h->plo[h->par] : nullptr, h->closing, h->acc_valid, h->nsm * 8, h->st);
   BONSAI_CUDA_TRY(cudaEventRecord(h->ev_in_consumed, h->st));
-  k_iota<<<h->nsm * 4, 256, 0, h->st>>>(h->id[h->par], n);
-  if (h->precision) BONSAI_CUDA_TRY(cudaMemsetAsync(h->plo[h->par], 0, bytes, h->st));
-  BONSAI_CUDA_TRY(cudaMemsetAsync(h->closing, 0, sizeof(int), h->st));
-  BONSAI_CUDA_TRY(cudaMemsetAsync(h->acc_valid, 0, 2 * sizeof(int), h->st));
   h->built = h->mp_done = h->grouped = h->forced = h->moved_after_forces = false;
   h->bts_ready = false;
   return last_cuda();
@@ -991,11 +1035,14 @@ int bonsai_get_particles_async(bonsai_handle hh, float* pos4, float* vel4, float
   float* dst[3] = {pos4, vel4, acc4};
   // the slot is free once its previous download has finished
   BONSAI_CUDA_TRY(cudaStreamWaitEvent(h->st, h->ev_out_done[slot], 0));
+  float4* out[3] = {nullptr, nullptr, nullptr};
   for (int a = 0; a < 3; a++) {
     if (!dst[a]) continue;
     if (!h->out_buf[slot][a]) BONSAI_CUDA_TRY(dalloc(&h->out_buf[slot][a], (size_t)n));
-    k_scatter_by_id<<<h->nsm * 8, 256, 0, h->st>>>(h->id[h->par], n, src[a], h->out_buf[slot][a]);
+    out[a] = h->out_buf[slot][a];
   }
+  launch_invert(h->id[h->par], n, h->valt, h->nsm * 8, h->st);
+  launch_fetch(h->valt, n, src, out, h->nsm * 8, h->st);
   BONSAI_CUDA_TRY(cudaEventRecord(h->ev_out_ready[slot], h->st));
   BONSAI_CUDA_TRY(cudaStreamWaitEvent(h->st_d2h, h->ev_out_ready[slot], 0));
   for (int a = 0; a < 3; a++)
