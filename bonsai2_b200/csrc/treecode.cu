@@ -182,18 +182,22 @@ struct Handle {
   // stage bookkeeping for the eager API
   bool built = false, mp_done = false, grouped = false, forced = false, moved_after_forces = false;
   bool ever_built = false, ever_mp = false;  // the cell arrays hold a tree / multipoles
-  // graphs, one per state parity and phase (0: build+multipoles+groups, 1: walk, 2: move)
+  // graphs of a step, one per state parity: gstep the whole step; gexec its
+  // phases (0: build+multipoles+groups, 1: walk, 2: move), for timed steps
+  cudaGraphExec_t gstep[2] = {nullptr, nullptr};
   cudaGraphExec_t gexec[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
   int graph_kernels = 0;
-  bool graph_ok = false;
+  bool graph_ok = false, phases_ok = false;
 
   ~Handle() { release(); }
 
   void release_graphs() {
-    for (int p = 0; p < 2; p++)
+    for (int p = 0; p < 2; p++) {
+      if (gstep[p]) { cudaGraphExecDestroy(gstep[p]); gstep[p] = nullptr; }
       for (int k = 0; k < 3; k++)
         if (gexec[p][k]) { cudaGraphExecDestroy(gexec[p][k]); gexec[p][k] = nullptr; }
-    graph_ok = false;
+    }
+    graph_ok = phases_ok = false;
   }
 
   void release_systems() {
@@ -615,45 +619,64 @@ struct Handle {
     }
   }
 
+  // the whole step (k < 0) or its phase k as a graph
+  int capture_one(int k, cudaGraphExec_t* exec, int* kernels) {
+    cudaGraph_t g = nullptr;
+    BONSAI_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    if (k < 0) enq_step(); else enq_phase(k);
+    cudaError_t e = cudaStreamEndCapture(st, &g);
+    if (e != cudaSuccess) return -(int)e - 1000;
+    if (kernels) {
+      size_t nn = 0;
+      cudaGraphGetNodes(g, nullptr, &nn);
+      std::vector<cudaGraphNode_t> nodes(nn);
+      cudaGraphGetNodes(g, nodes.data(), &nn);
+      for (size_t q = 0; q < nn; q++) {
+        cudaGraphNodeType ty;
+        cudaGraphNodeGetType(nodes[q], &ty);
+        *kernels += (ty == cudaGraphNodeTypeKernel);
+      }
+    }
+    e = cudaGraphInstantiate(exec, g, 0);
+    cudaGraphDestroy(g);
+    return e == cudaSuccess ? 0 : -(int)e - 1000;
+  }
   int capture_graphs() {
     release_graphs();
     const int par0 = par;
     graph_kernels = 0;
-    for (int p = 0; p < 2; p++) {
+    int rc = 0;
+    for (int p = 0; p < 2 && !rc; p++) {
       par = p;
-      for (int k = 0; k < 3; k++) {
-        cudaGraph_t g = nullptr;
-        BONSAI_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        enq_phase(k);
-        cudaError_t e = cudaStreamEndCapture(st, &g);
-        if (e != cudaSuccess) { par = par0; return -(int)e - 1000; }
-        if (p == 0) {
-          size_t nn = 0;
-          cudaGraphGetNodes(g, nullptr, &nn);
-          std::vector<cudaGraphNode_t> nodes(nn);
-          cudaGraphGetNodes(g, nodes.data(), &nn);
-          for (size_t q = 0; q < nn; q++) {
-            cudaGraphNodeType ty;
-            cudaGraphNodeGetType(nodes[q], &ty);
-            graph_kernels += (ty == cudaGraphNodeTypeKernel);
-          }
-        }
-        e = cudaGraphInstantiate(&gexec[p][k], g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) { par = par0; return -(int)e - 1000; }
-      }
+      rc = capture_one(-1, &gstep[p], p == 0 ? &graph_kernels : nullptr);
     }
     par = par0;
-    graph_ok = true;
-    return 0;
+    graph_ok = rc == 0;
+    return rc;
+  }
+  int capture_phases() {
+    const int par0 = par;
+    int rc = 0;
+    for (int p = 0; p < 2 && !rc; p++) {
+      par = p;
+      for (int k = 0; k < 3 && !rc; k++) rc = capture_one(k, &gexec[p][k], nullptr);
+    }
+    par = par0;
+    phases_ok = rc == 0;
+    return rc;
   }
 
+  // ev: four events around the phases, or null for the whole step at once
   int launch_graph_step(cudaEvent_t* ev) {
-    for (int k = 0; k < 3; k++) {
-      if (ev) BONSAI_CUDA_TRY(cudaEventRecord(ev[k], st));
-      BONSAI_CUDA_TRY(cudaGraphLaunch(gexec[par][k], st));
+    if (!ev) {
+      BONSAI_CUDA_TRY(cudaGraphLaunch(gstep[par], st));
+    } else {
+      for (int k = 0; k < 3; k++) {
+        BONSAI_CUDA_TRY(cudaEventRecord(ev[k], st));
+        BONSAI_CUDA_TRY(cudaGraphLaunch(gexec[par][k], st));
+      }
+      BONSAI_CUDA_TRY(cudaEventRecord(ev[3], st));
     }
-    if (ev) BONSAI_CUDA_TRY(cudaEventRecord(ev[3], st));
     par ^= 1;
     return 0;
   }
@@ -1176,6 +1199,10 @@ int bonsai_step_timed(bonsai_handle hh, int nsteps, float* phase_ms) {
     int rc = h->build_checked(h->cur_nleaf);
     if (rc) return rc;
     rc = h->capture_graphs();
+    if (rc) return rc;
+  }
+  if (!h->phases_ok) {
+    const int rc = h->capture_phases();
     if (rc) return rc;
   }
   std::vector<cudaEvent_t> ev((size_t)4 * nsteps);
