@@ -172,7 +172,14 @@ __device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned round, in
   return ok != 0;
 }
 
-template <bool DS>
+// Barrier of the level launch: the one block, the one cluster, or the grid.
+enum LevelGroup { kOneBlock, kOneCluster, kWholeGrid };
+constexpr int kLvCluster = 8;
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+template <bool DS, LevelGroup G>
 __global__ void __launch_bounds__(kLvThreads, kLvMaxBlocksPerSm)
     k_mp_levels(TreeInfo* __restrict__ info, const uint4* __restrict__ cell_data, float inv_theta, MpRec* rec,
                 typename BoxOf<DS>::T* box, float4* __restrict__ cell_open, float4* __restrict__ cell_stage,
@@ -188,10 +195,10 @@ __global__ void __launch_bounds__(kLvThreads, kLvMaxBlocksPerSm)
   const int top = info->nlevels - 1;
   for (int L = top; L >= 1; L--) {
     const int b = info->level_beg[L], e = info->level_end[L];
-    // A narrow level is the first block's alone, and between two narrow levels
-    // the block's own barrier will do: a grid-wide one, about as long as the
-    // level itself, is taken only before a wide level and after it.
-    const bool narrow = e - b <= kNarrow;
+    // A narrow level of a grid is the first block's alone, and between two
+    // narrow levels the block's own barrier will do: a grid-wide one, about as
+    // long as the level itself, is taken only before a wide level and after it.
+    const bool narrow = G == kWholeGrid && e - b <= kNarrow;
     // cells a warp looks at together: fewer where the level would leave warps idle
     const int nw = narrow ? kLvWarps : nwarps;
     int span = 4;
@@ -200,9 +207,15 @@ __global__ void __launch_bounds__(kLvThreads, kLvMaxBlocksPerSm)
     // the first cells' words do not wait for the level below
     unsigned yl = (lane < span && cfirst + lane < e) ? __ldg(&cell_data[cfirst + lane].y) : 0xFFFFFFFFu;
     if (L < top) {
-      const bool below = info->level_end[L + 1] - info->level_beg[L + 1] <= kNarrow;
-      if (narrow && below) __syncthreads();
-      else if (!grid_barrier(barrier, ++round, &info->status)) return;
+      if (G == kOneBlock) {
+        __syncthreads();
+      } else if (G == kOneCluster) {
+        cluster_barrier();
+      } else {
+        const bool below = info->level_end[L + 1] - info->level_beg[L + 1] <= kNarrow;
+        if (narrow && below) __syncthreads();
+        else if (!grid_barrier(barrier, ++round, &info->status)) return;
+      }
     }
     if (narrow && blockIdx.x != 0) continue;
     for (int c0 = cfirst; c0 < e; c0 += nw * span) {
@@ -331,15 +344,7 @@ __global__ void __launch_bounds__(256) k_multipoles(const int* __restrict__ leaf
     // one pass: sums about the leaf's first particle x0 (d = x - x0), then the
     // shift to the centre of mass: COM = x0 + S1/M, I = S2 - S1 S1^T / M; the
     // cancellation is relative to the leaf's extent, not to |x0|
-    double x0, y0, z0;
-    {
-      const float4 p = __ldg(jpos + b);
-      x0 = p.x; y0 = p.y; z0 = p.z;
-      if (DS) {
-        const float4 l = __ldg(jlo + b);
-        x0 += l.x; y0 += l.y; z0 += l.z;
-      }
-    }
+    double x0 = 0, y0 = 0, z0 = 0;
     double m = 0, s1x = 0, s1y = 0, s1z = 0, q[6] = {0, 0, 0, 0, 0, 0};
     // four particles' loads in flight before they are summed (in order)
     for (int i0 = b; i0 < e; i0 += kMpBatch) {
@@ -349,6 +354,10 @@ __global__ void __launch_bounds__(256) k_multipoles(const int* __restrict__ leaf
         const int i = min(i0 + u, e - 1);
         pb[u] = __ldg(jpos + i);
         if (DS) lb[u] = __ldg(jlo + i);
+      }
+      if (i0 == b) {
+        x0 = pb[0].x; y0 = pb[0].y; z0 = pb[0].z;
+        if (DS) { x0 += lb[0].x; y0 += lb[0].y; z0 += lb[0].z; }
       }
 #pragma unroll
       for (int u = 0; u < kMpBatch; u++) {
@@ -430,13 +439,17 @@ __global__ void __launch_bounds__(256) k_multipoles(const int* __restrict__ leaf
   }
 }
 
+// One block up to 2048 particles, a cluster of eight (its hardware barrier) up to
+// 16,384, above that the grid: build of 4096 particles 100 -> 94 us against the
+// grid, 16,384 126.5 -> 124.4, 30,011 129 -> 141 (eight blocks are too few).
+constexpr int kClusterMin = 2048, kClusterMax = 16384;
 constexpr int kLvSmem = kLvWarps * 4 * kNodeDoubles * (int)sizeof(double);
 
 // blocks of the level launch that are resident at once
 int multipole_level_blocks(int nsm) {
   int a = 0, b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_mp_levels<false>, kLvThreads, kLvSmem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_mp_levels<true>, kLvThreads, kLvSmem) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_mp_levels<false, kWholeGrid>, kLvThreads, kLvSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_mp_levels<true, kWholeGrid>, kLvThreads, kLvSmem) != cudaSuccess)
     return 1;
   return std::max(1, nsm * std::min(std::min(a, b), kLvMaxBlocksPerSm));
 }
@@ -448,12 +461,34 @@ static void launch_multipoles_of(const int* leaf_list, TreeInfo* info, const uin
                                  float4* cell_lo, int nblocks, unsigned* barrier, int level_blocks, cudaStream_t s) {
   k_multipoles<DS><<<nblocks, 256, 0, s>>>(leaf_list, info, cell_data, jpos, inv_theta, rec, box, cell_open,
                                            cell_stage, cell_ls, cell_cap, jlo, cell_lo, barrier);
-  // about 1024 particles per block: more give the widest level its teams, fewer
-  // make the barrier cheaper
-  int grid = std::min(level_blocks, std::max(1, n / 1024));
-  void* args[] = {&info, &cell_data, &inv_theta, &rec, &box, &cell_open, &cell_stage, &cell_ls, &cell_cap, &cell_lo,
-                  &barrier};
-  cudaLaunchCooperativeKernel((const void*)k_mp_levels<DS>, dim3(grid), dim3(kLvThreads), args, (size_t)kLvSmem, s);
+  if (n <= kClusterMin) {
+    k_mp_levels<DS, kOneBlock><<<1, kLvThreads, kLvSmem, s>>>(info, cell_data, inv_theta, rec, box, cell_open,
+                                                              cell_stage, cell_ls, cell_cap, cell_lo, barrier);
+    return;
+  }
+  cudaLaunchAttribute at[1];
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kLvThreads);
+  cfg.dynamicSmemBytes = kLvSmem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (n <= kClusterMax) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kLvCluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(kLvCluster);
+    cudaLaunchKernelEx(&cfg, k_mp_levels<DS, kOneCluster>, info, cell_data, inv_theta, rec, box, cell_open, cell_stage,
+                       cell_ls, cell_cap, cell_lo, barrier);
+  } else {
+    // about 1024 particles per block: more give the widest level its teams, fewer
+    // make the barrier cheaper
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.gridDim = dim3(std::min(level_blocks, n / 1024));
+    cudaLaunchKernelEx(&cfg, k_mp_levels<DS, kWholeGrid>, info, cell_data, inv_theta, rec, box, cell_open, cell_stage,
+                       cell_ls, cell_cap, cell_lo, barrier);
+  }
 }
 
 void launch_multipoles(const int* leaf_list, TreeInfo* info, const uint4* cell_data, const float4* jpos, int n,

@@ -1524,7 +1524,7 @@ const char* bonsai_error_string(int code) {
     if (code & BONSAI_STATUS_GROUP_CAPACITY) return "group capacity exceeded";
     if (code & BONSAI_STATUS_DEPTH) return "tree deeper than 21 levels (fat leaf kept)";
     if (code & BONSAI_STATUS_BAD_PARAM) return "bad parameter";
-    if (code & BONSAI_STATUS_SORT_TIMEOUT) return "radix sort look-back wait timed out";
+    if (code & BONSAI_STATUS_SORT_TIMEOUT) return "device wait (radix sort look-back or multipole level barrier) timed out";
     if (code & BONSAI_STATUS_BOUNDS) return "index out of range (bounds-checked build; access skipped)";
   }
   return "unknown";

@@ -35,7 +35,7 @@ extern "C" {
 #define BONSAI_STATUS_NONFINITE 8      /* NaN/Inf coordinate in the input */
 #define BONSAI_STATUS_GROUP_CAPACITY 16
 #define BONSAI_STATUS_BAD_PARAM 32
-#define BONSAI_STATUS_SORT_TIMEOUT 64  /* a radix-sort look-back wait hit its bound: results invalid */
+#define BONSAI_STATUS_SORT_TIMEOUT 64  /* a device wait (radix-sort look-back, multipole level barrier) hit its bound: results invalid */
 #define BONSAI_STATUS_BOUNDS 128       /* bounds-checked build only: a guarded index was out of range (access skipped) */
 
 /* API errors */
