@@ -1646,7 +1646,7 @@ int bonsai_direct_fp64(bonsai_handle hh, const int* sample, int ns, int include_
   for (int s = 0; s < ns; s++)
     if (sample[s] < 0 || sample[s] >= h->n) return BONSAI_ERR_ARG;
   BONSAI_CUDA_TRY(cudaSetDevice(h->dev));
-  const int nsplit = std::max(1, std::min(512, (h->nsm * 8 * 256) / std::max(ns, 1)));
+  const int nsplit = direct_slices(ns, h->nsm);
   if (ns > h->direct_cap || !h->direct_part) {
     dfree(&h->direct_part); dfree(&h->direct_out); dfree(&h->direct_sample);
     BONSAI_CUDA_TRY(dalloc(&h->direct_part, (size_t)512 * ns * 4));
