@@ -162,6 +162,10 @@ __global__ void k_scatter_by_id(const int* __restrict__ id, int n, const float4*
                                 float4* __restrict__ out);
 void launch_load_state(const float4* pos, const float4* vel, int n, float4* pos_o, float4* vel_o, int* id, float4* lo,
                        int* closing, int* acc_valid, int nblocks, cudaStream_t s);
+// double positions in (records first .. first + count of the particles) and out, in the caller's order
+void launch_split_f64(const double* in, int first, int count, float4* pos, float4* lo, int nblocks, cudaStream_t s);
+void launch_join_f64(const int* inv, int n, int first, int count, const float4* pos, const float4* lo, double* out,
+                     int nblocks, cudaStream_t s);
 void launch_invert(const int* id, int n, int* inv, int nblocks, cudaStream_t s);
 // arrays in state order to the caller's order through inv (launch_invert); any dst may be null
 void launch_fetch(const int* inv, int n, const float4* const src[3], float4* const dst[3], int nblocks,

@@ -525,6 +525,46 @@ void launch_load_state(const float4* pos, const float4* vel, int n, float4* pos_
                                                                   acc_valid);
 }
 
+// Double positions (x, y, z, m), records first .. first + count of the
+// particles: hi = (float)x and, with lo, lo = (float)(x - hi).
+__global__ void __launch_bounds__(256) k_split_f64(const double2* __restrict__ in, int first, int count,
+                                                   float4* __restrict__ pos, float4* __restrict__ lo) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
+    const double2 a = __ldcs(in + 2 * (size_t)k), b = __ldcs(in + 2 * (size_t)k + 1);
+    const float4 h = make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
+    pos[first + k] = h;
+    if (lo)
+      lo[first + k] = make_float4((float)(a.x - (double)h.x), (float)(a.y - (double)h.y), (float)(b.x - (double)h.z), 0.f);
+  }
+}
+
+// the caller's particles first .. first + count as doubles hi + lo, through inv
+__global__ void __launch_bounds__(256) k_join_f64(const int* __restrict__ inv, int n, int first, int count,
+                                                  const float4* __restrict__ pos, const float4* __restrict__ lo,
+                                                  double2* __restrict__ out) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
+    const int j = __ldcs(inv + first + k);
+    if ((unsigned)j >= (unsigned)n) continue;  // (no particles loaded)
+    const float4 h = __ldg(pos + j);
+    float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lo) l = __ldg(lo + j);
+    __stcs(out + 2 * (size_t)k, make_double2((double)h.x + (double)l.x, (double)h.y + (double)l.y));
+    __stcs(out + 2 * (size_t)k + 1, make_double2((double)h.z + (double)l.z, (double)h.w));
+  }
+}
+
+void launch_split_f64(const double* in, int first, int count, float4* pos, float4* lo, int nblocks, cudaStream_t s) {
+  if (count > 0)
+    k_split_f64<<<std::min(nblocks, (count + 255) / 256), 256, 0, s>>>(reinterpret_cast<const double2*>(in), first,
+                                                                       count, pos, lo);
+}
+void launch_join_f64(const int* inv, int n, int first, int count, const float4* pos, const float4* lo, double* out,
+                     int nblocks, cudaStream_t s) {
+  if (count > 0)
+    k_join_f64<<<std::min(nblocks, (count + 255) / 256), 256, 0, s>>>(inv, n, first, count, pos, lo,
+                                                                      reinterpret_cast<double2*>(out));
+}
+
 // inv[id[k]] = k
 __global__ void __launch_bounds__(256) k_invert(const int* __restrict__ id, int n, int* __restrict__ inv) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {

@@ -117,6 +117,7 @@ struct Handle {
   unsigned long long* stats = nullptr;
   double *move_partial = nullptr, *energies = nullptr;
   unsigned *move_ticket = nullptr, *box_ticket = nullptr;
+  double* f64_odd = nullptr;  // one double position (bonsai_set_particles_f64)
   unsigned* mp_barrier = nullptr;  // of the multipoles' level launch
   int mp_level_blocks = 1;
   int* closing = nullptr;
@@ -277,7 +278,7 @@ struct Handle {
     release_particles();
     dfree(&info); dfree(&g_count); dfree(&g_seg); dfree(&g_ng); dfree(&ring);
     dfree(&group_counter); dfree(&stats); dfree(&move_partial); dfree(&energies);
-    dfree(&move_ticket); dfree(&box_ticket); dfree(&mp_barrier); dfree(&order_count); dfree(&closing); dfree(&acc_valid); dfree(&box); dfree(&box_partial);
+    dfree(&move_ticket); dfree(&box_ticket); dfree(&mp_barrier); dfree(&f64_odd); dfree(&order_count); dfree(&closing); dfree(&acc_valid); dfree(&box); dfree(&box_partial);
     dfree(&ph_table); dfree(&direct_part); dfree(&direct_out); dfree(&direct_sample);
     dfree(&mlp_w);
     if (mlp_wh) { cudaFree(mlp_wh); mlp_wh = nullptr; }
@@ -349,6 +350,7 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&move_ticket, 1));
     BONSAI_CUDA_TRY(dalloc(&box_ticket, 1));
     BONSAI_CUDA_TRY(dalloc(&mp_barrier, 1));
+    BONSAI_CUDA_TRY(dalloc(&f64_odd, 4));
     BONSAI_CUDA_TRY(dalloc(&order_count, 2));
     mp_level_blocks = multipole_level_blocks(nsm);
     BONSAI_CUDA_TRY(cudaMemset(move_ticket, 0, sizeof(unsigned)));
@@ -1260,22 +1262,43 @@ int bonsai_set_precision(bonsai_handle hh, int mode) {
   return h->alloc_lo();
 }
 
+// Double positions cross the bus as they are and are split and joined on the
+// device, through the two idle state buffers: half of the particles (32 bytes
+// each) in each, and an odd one by itself.
+struct F64Part {
+  double* stage;
+  int first, count;
+};
+static F64Part f64_part(Handle* h, int c) {
+  const int half = h->n / 2;
+  if (c == 0) return {reinterpret_cast<double*>(h->pos[h->par ^ 1]), 0, half};
+  if (c == 1) return {reinterpret_cast<double*>(h->vel[h->par ^ 1]), half, half};
+  return {h->f64_odd, 2 * half, h->n - 2 * half};
+}
+
 int bonsai_set_particles_f64(bonsai_handle hh, const double* pos4, const float* vel4, int n) {
   Handle* h = H(hh);
   if (!h) return BONSAI_ERR_HANDLE;
   if (!pos4 || !vel4 || n < 1) return BONSAI_ERR_ARG;
-  const size_t N = (size_t)n;
-  std::vector<float4> hi(N), lo(N);
-  for (size_t i = 0; i < N; i++) {
-    const double x = pos4[4 * i], y = pos4[4 * i + 1], z = pos4[4 * i + 2];
-    hi[i] = make_float4((float)x, (float)y, (float)z, (float)pos4[4 * i + 3]);
-    lo[i] = make_float4((float)(x - (double)hi[i].x), (float)(y - (double)hi[i].y), (float)(z - (double)hi[i].z), 0.f);
+  BONSAI_CUDA_TRY(cudaSetDevice(h->dev));
+  if (n != h->n) {
+    const int rc = h->alloc(n);
+    if (rc) return rc;
   }
-  int rc = set_particles_impl(h, &hi[0].x, vel4, n, cudaMemcpyHostToDevice);
-  if (rc) return rc;
-  if (h->precision)
-    BONSAI_CUDA_TRY(cudaMemcpyAsync(h->plo[h->par], lo.data(), N * sizeof(float4), cudaMemcpyHostToDevice, h->st));
-  BONSAI_CUDA_TRY(cudaStreamSynchronize(h->st));  // the host staging vectors go out of scope
+  BONSAI_CUDA_TRY(cudaMemcpyAsync(h->vel[h->par], vel4, (size_t)n * sizeof(float4), cudaMemcpyHostToDevice, h->st));
+  launch_load_state(nullptr, nullptr, n, h->pos[h->par], h->vel[h->par], h->id[h->par], nullptr, h->closing,
+                    h->acc_valid, h->nsm * 8, h->st);
+  for (int c = 0; c < 3; c++) {
+    const F64Part q = f64_part(h, c);
+    if (q.count == 0) continue;
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(q.stage, pos4 + 4 * (size_t)q.first, (size_t)q.count * 4 * sizeof(double),
+                                    cudaMemcpyHostToDevice, h->st));
+    launch_split_f64(q.stage, q.first, q.count, h->pos[h->par], h->precision ? h->plo[h->par] : nullptr, h->nsm * 8,
+                     h->st);
+  }
+  h->built = h->mp_done = h->grouped = h->forced = h->moved_after_forces = false;
+  h->bts_ready = false;
+  BONSAI_CUDA_TRY(cudaStreamSynchronize(h->st));
   return last_cuda();
 }
 
@@ -1283,24 +1306,18 @@ int bonsai_get_particles_f64(bonsai_handle hh, double* pos4, float* vel4, float*
   Handle* h = H(hh);
   if (!h) return BONSAI_ERR_HANDLE;
   if (h->n == 0) return BONSAI_ERR_NOT_ALLOCATED;
-  int rc = get_particles_impl(h, nullptr, vel4, acc4, cudaMemcpyDeviceToHost);
+  const int rc = get_particles_impl(h, nullptr, vel4, acc4, cudaMemcpyDeviceToHost);
   if (rc || !pos4) return rc;
-  const size_t N = (size_t)h->n;
-  std::vector<float4> hi(N), lo(N, make_float4(0.f, 0.f, 0.f, 0.f));
-  rc = get_particles_impl(h, &hi[0].x, nullptr, nullptr, cudaMemcpyDeviceToHost);
-  if (rc) return rc;
-  if (h->precision) {
-    float4* tmp = h->pos[h->par ^ 1];
-    k_scatter_by_id<<<h->nsm * 8, 256, 0, h->st>>>(h->id[h->par], h->n, h->plo[h->par], tmp);
-    BONSAI_CUDA_TRY(cudaMemcpyAsync(lo.data(), tmp, N * sizeof(float4), cudaMemcpyDeviceToHost, h->st));
-    BONSAI_CUDA_TRY(cudaStreamSynchronize(h->st));
+  launch_invert(h->id[h->par], h->n, h->valt, h->nsm * 8, h->st);
+  for (int c = 0; c < 3; c++) {
+    const F64Part q = f64_part(h, c);
+    if (q.count == 0) continue;
+    launch_join_f64(h->valt, h->n, q.first, q.count, h->pos[h->par], h->precision ? h->plo[h->par] : nullptr, q.stage,
+                    h->nsm * 8, h->st);
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(pos4 + 4 * (size_t)q.first, q.stage, (size_t)q.count * 4 * sizeof(double),
+                                    cudaMemcpyDeviceToHost, h->st));
   }
-  for (size_t i = 0; i < N; i++) {
-    pos4[4 * i] = (double)hi[i].x + (double)lo[i].x;
-    pos4[4 * i + 1] = (double)hi[i].y + (double)lo[i].y;
-    pos4[4 * i + 2] = (double)hi[i].z + (double)lo[i].z;
-    pos4[4 * i + 3] = (double)hi[i].w;
-  }
+  BONSAI_CUDA_TRY(cudaStreamSynchronize(h->st));
   return last_cuda();
 }
 

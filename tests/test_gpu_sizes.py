@@ -123,3 +123,25 @@ def test_device_arrays(lib, n, shift):
     assert lib.bonsai_get_particles_device(t.handle, None, None, ptr[4]) == 0
     assert np.array_equal(part[4].cpu().numpy().reshape(n, 4), acc)
     t.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 4097, 70000])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_double_positions_round_trip(lib, n, precision):
+    """Positions split into float pairs on the device and joined again: exactly
+    what the same split gives on the host, for even and odd counts."""
+    import bonsai2_b200 as B
+    rng = np.random.default_rng(n)
+    pos = np.column_stack([rng.normal(size=(n, 3)) * 10.0 ** rng.uniform(-6, 6, (n, 1)), rng.uniform(0.1, 1, n)])
+    vel = rng.normal(size=(n, 4)).astype(np.float32)
+    t = B.Treecode()
+    t.alloc(n)
+    t.set_precision(precision)
+    t.set_particles_f64(pos, vel)
+    p, v, _ = t.get_particles_f64()
+    hi = pos.astype(np.float32)
+    want = hi.astype(np.float64)
+    if precision:
+        want[:, :3] += (pos[:, :3] - want[:, :3]).astype(np.float32)
+    assert np.array_equal(p, want) and np.array_equal(v, vel)
+    t.close()
