@@ -267,7 +267,7 @@ __global__ void k_fill_inv_theta(const TreeInfo* __restrict__ info, const float*
 // All of it is FP32.  64 samples per block give 128 blocks at S = 8192 (one
 // wave on 148 SMs); more per block would leave SMs idle.  Bound by the one
 // tile's own chain (weights staged, three products, tanh, gradients) at that
-// size: 17.2 us, and 3.0 us for the fold (one B200).  The form it replaced kept
+// size: 16.2 us, and 3.0 us for the fold (one B200).  The form it replaced kept
 // activations in global memory, one warp per sample, and summed each weight's
 // gradient by one thread's serial loop over its samples: 27 + 67 + 2.3 + 1.9
 // us an epoch.  100 epochs through the entry point: 13.0 -> 3.2 ms.
@@ -279,7 +279,8 @@ constexpr int kXRow = kF + 4;
 // shared memory, in floats: W1 and W2 input-major for the forward products,
 // W2 as it is for the backward one, biases and w3; then the tile's x, h1, d2,
 // d1 (after the last tile the same space folds the gradients)
-constexpr int sW1t = 0, sW2t = sW1t + kF * kH, sW2 = sW2t + kH * kH, sB1 = sW2 + kH * kH, sB2 = sB1 + kH,
+// (transposed rows padded, so that the strided writes fall on 8 banks, not one)
+constexpr int sW1t = 0, sW2t = sW1t + kF * kRow, sW2 = sW2t + kH * kRow, sB1 = sW2 + kH * kH, sB2 = sB1 + kH,
               sW3 = sB2 + kH, sX = sW3 + kH, sH1 = sX + kTS * kXRow, sD2 = sH1 + kTS * kRow,
               sD1 = sD2 + kTS * kRow, kEpochFloats = sD1 + kTS * kRow;
 
@@ -289,7 +290,7 @@ __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z,
 __device__ __forceinline__ float comp(const float4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
 
 // acc[u] (u = sample, 4 units as two pairs) += sum_k a[s + u][k] * w[k][4 units]
-template <int K>
+template <int K, int WROW>
 __device__ __forceinline__ void tile_product(const float* a, int arow, const float* w, float2 (&acc)[2][2]) {
 #pragma unroll 4
   for (int k0 = 0; k0 < K; k0 += 4) {
@@ -297,7 +298,7 @@ __device__ __forceinline__ void tile_product(const float* a, int arow, const flo
     const float4 a1 = *reinterpret_cast<const float4*>(a + arow + k0);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const float4 v = *reinterpret_cast<const float4*>(w + (k0 + k) * kH);
+      const float4 v = *reinterpret_cast<const float4*>(w + (k0 + k) * WROW);
       acc[0][0] = __ffma2_rn(dup2(comp(a0, k)), lo2(v), acc[0][0]);
       acc[0][1] = __ffma2_rn(dup2(comp(a0, k)), hi2(v), acc[0][1]);
       acc[1][0] = __ffma2_rn(dup2(comp(a1, k)), lo2(v), acc[1][0]);
@@ -315,11 +316,11 @@ __global__ void __launch_bounds__(kEpochThreads, 1)
   extern __shared__ float4 smem4[];
   float* sm = reinterpret_cast<float*>(smem4);
   const int t = threadIdx.x;
-  for (int i = t; i < kH * kF; i += kEpochThreads) sm[sW1t + (i % kF) * kH + i / kF] = w[oW1 + i];
+  for (int i = t; i < kH * kF; i += kEpochThreads) sm[sW1t + (i % kF) * kRow + i / kF] = w[oW1 + i];
   for (int i = t; i < kH * kH; i += kEpochThreads) {
     const float v = w[oW2 + i];
     sm[sW2 + i] = v;
-    sm[sW2t + (i % kH) * kH + i / kH] = v;
+    sm[sW2t + (i % kH) * kRow + i / kH] = v;
   }
   if (t < kH) { sm[sB1 + t] = w[oB1 + t]; sm[sB2 + t] = w[oB2 + t]; sm[sW3 + t] = w[oW3 + t]; }
   const float b3 = w[oB3];
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(kEpochThreads, 1)
     const float4 bb1 = *reinterpret_cast<const float4*>(sm + sB1 + u0);
 #pragma unroll
     for (int u = 0; u < 2; u++) { a[u][0] = lo2(bb1); a[u][1] = hi2(bb1); }
-    tile_product<kF>(sm + sX + r0 * kXRow, kXRow, sm + sW1t + u0, a);
+    tile_product<kF, kRow>(sm + sX + r0 * kXRow, kXRow, sm + sW1t + u0, a);
     float h1[2][4];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(kEpochThreads, 1)
     const float4 bb2 = *reinterpret_cast<const float4*>(sm + sB2 + u0);
 #pragma unroll
     for (int u = 0; u < 2; u++) { a[u][0] = lo2(bb2); a[u][1] = hi2(bb2); }
-    tile_product<kH>(sm + sH1 + r0 * kRow, kRow, sm + sW2t + u0, a);
+    tile_product<kH, kRow>(sm + sH1 + r0 * kRow, kRow, sm + sW2t + u0, a);
     const float4 w3 = *reinterpret_cast<const float4*>(sm + sW3 + u0);
 #pragma unroll
     for (int u = 0; u < 2; u++) {
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(kEpochThreads, 1)
     if (BACK) {
       __syncwarp();
       a[0][0] = a[0][1] = a[1][0] = a[1][1] = dup2(0.f);
-      tile_product<kH>(sm + sD2 + r0 * kRow, kRow, sm + sW2 + u0, a);
+      tile_product<kH, kH>(sm + sD2 + r0 * kRow, kRow, sm + sW2 + u0, a);
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         const float v[4] = {a[u][0].x, a[u][0].y, a[u][1].x, a[u][1].y};
