@@ -582,6 +582,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
 
         // (3) particles of opened leaves -> direct ring
         const int nb = (split && leaf) ? (int)(cd.w - cd.z) : 0;
+        if (!__any_sync(kFull, nb)) continue;
         const int incl2 = warp_incl_scan(nb);
         const int tot2 = __shfl_sync(kFull, incl2, 31);
         const int pb = (int)cd.z;
