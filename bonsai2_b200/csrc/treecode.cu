@@ -789,16 +789,21 @@ struct Handle {
     }
     const int nsub = 1 << bts_K;
     int maxl = bts_K;
+    bool stale = true;
     for (int b = 0; b < nsteps; b++) {
       for (int s = 0; s < nsub; s++) {
         lo_p = precision ? plo[par] : nullptr;
         launch_bts_open_drift(pos[par], vel[par], acc, lev[par], n, prm.dt, bts_K, s, lo_p, nb, st);
         // the particles ending at s + 1 have level >= K - tz(s + 1); when none
         // is that fine, the substep is the drift alone (nothing else changes)
+        // (levels change where steps end: the largest is read after that)
         if (bts_K > 0 && s + 1 < nsub) {
-          launch_max_level(lev[par], n, max_lev, nb, st);
-          BONSAI_CUDA_TRY(cudaMemcpyAsync(&maxl, max_lev, sizeof(int), cudaMemcpyDeviceToHost, st));
-          BONSAI_CUDA_TRY(cudaStreamSynchronize(st));
+          if (stale) {
+            launch_max_level(lev[par], n, max_lev, nb, st);
+            BONSAI_CUDA_TRY(cudaMemcpyAsync(&maxl, max_lev, sizeof(int), cudaMemcpyDeviceToHost, st));
+            BONSAI_CUDA_TRY(cudaStreamSynchronize(st));
+            stale = false;
+          }
           if (maxl < bts_K - (__builtin_ctz((unsigned)(s + 1)))) continue;
         }
         enq_build_groups(cur_nleaf, cur_ls, cur_ncrit);
@@ -807,6 +812,7 @@ struct Handle {
         enq_forces(cur_ncrit);
         walk_list_on = false;
         launch_bts_close(vel[par], acc, lev[par], n, prm.dt, bts_K, s + 1, bts_eta, prm.eps, 0, nb, st);
+        stale = true;
       }
       // energies at the synchronised end of the big step (closing flag is 0)
       enq_move(false);
