@@ -147,7 +147,7 @@ constexpr int kLvMaxBlocksPerSm = 2;
 // nodes of a half-warp fall on other banks
 constexpr int kNodeDoubles = 81;
 constexpr int kNarrow = 256;  // cells of a level that one block takes (64 teams)
-constexpr int kBarrierSpin = 1 << 24;
+constexpr int kBarrierSpin = 1 << 22;  // a few seconds
 
 // All blocks have arrived `round` times.  The wait is bounded: past the bound
 // it reports, and the caller returns (results invalid).

@@ -145,3 +145,41 @@ def test_double_positions_round_trip(lib, n, precision):
         want[:, :3] += (pos[:, :3] - want[:, :3]).astype(np.float32)
     assert np.array_equal(p, want) and np.array_equal(v, vel)
     t.close()
+
+
+def test_handles_in_threads(lib):
+    """Handles stepped from threads of their own at once give what each gives
+    alone: their steps share the GPU, grid-wide barriers of the multipoles'
+    level launches among them."""
+    import threading
+
+    import bonsai2_b200 as B
+    sizes = [300007, 40000, 300007, 150001, 9000]
+    steps = 12
+
+    inputs = [B.plummer(n, k + 1) for k, n in enumerate(sizes)]  # (one rand() stream: not in the threads)
+
+    def run(n, out, k):
+        pos, vel = inputs[k]
+        t = B.Treecode(eps=0.01, theta=0.8)
+        t.alloc(n)
+        t.h_ptclPos[:] = pos
+        t.h_ptclVel[:] = vel
+        t.ptcl_h2d()
+        t.step(steps)
+        status = t.synchronize()
+        t.ptcl_d2h()
+        out[k] = (status, t.h_ptclPos.copy(), t.get_acc())
+        t.close()
+
+    alone, together = {}, {}
+    for k, n in enumerate(sizes):
+        run(n, alone, k)
+    threads = [threading.Thread(target=run, args=(n, together, k)) for k, n in enumerate(sizes)]
+    for x in threads:
+        x.start()
+    for x in threads:
+        x.join()
+    for k in range(len(sizes)):
+        assert alone[k][0] == 0 and together[k][0] == 0
+        assert np.array_equal(alone[k][1], together[k][1]) and np.array_equal(alone[k][2], together[k][2])
