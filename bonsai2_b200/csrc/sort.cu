@@ -20,14 +20,14 @@ namespace bonsai {
 
 constexpr int kSortThreads = 256;
 constexpr int kScanChunk = 4096;
-// Keys per thread of a one-sweep tile: 4 (1024-key tiles) while one wave of
-// tiles holds all keys, where a pass is one tile's latency (30,011 keys: 6.1 us
-// against 11); 16 above, where the digit runs that a tile writes out are longer
-// (2^20 keys, two sorts at once: 27 us either way; more tiles mean more look-back
-// words).  Same order either way.
-constexpr int kSmallItems = 4, kLargeItems = 16;
-constexpr int kSortSmallMax = 1 << 19;
-static int sort_items(int n) { return n <= kSortSmallMax ? kSmallItems : kLargeItems; }
+// Keys per thread of a one-sweep tile: 4 (1024-key tiles) where a pass is one
+// tile's latency, 16 where the digit runs that a tile writes out have to be long,
+// 8 between.  Build of a whole step with 4 / 8 / 16 (us): 30,011 particles 126 /
+// 139, 131,072 169 / 171 / 200, 250,007 220 / 212 / 229, 500,000 300 / 297 / 308,
+// 2^20 - / 413 / 450, 1.7M - / 591 / 571.  Same order with any.
+constexpr int kSmallItems = 4, kMidItems = 8, kLargeItems = 16;
+constexpr int kSortSmallMax = 1 << 17, kSortMidMax = 1 << 20;
+static int sort_items(int n) { return n <= kSortSmallMax ? kSmallItems : (n <= kSortMidMax ? kMidItems : kLargeItems); }
 
 int sort_tiles(int n) {
   const int tile = kSortThreads * sort_items(n);
@@ -125,7 +125,7 @@ void exclusive_scan(const unsigned* in, unsigned* out, int m, unsigned* bsum, un
 // ---------------------------------------------------------------------------
 // One-sweep passes.  One kernel reads the keys once and builds the digit
 // histograms of all eight passes; one kernel per pass then ranks each
-// 4096-key tile (same stable warp ranking as above), obtains the tile's
+// tile (the same stable warp ranking for every tile size), obtains the tile's
 // global offset per digit by decoupled look-back over the preceding tiles
 // (tiles take ids in launch order from an atomic counter, so a tile only waits
 // for tiles that already run; every wait is bounded and sets an error flag
@@ -477,6 +477,8 @@ void radix_sort_pairs(unsigned long long* keys_a, unsigned long long* keys_b, in
     k_sort_block<<<1, threads, kOneSmem, s>>>(keys_a, vals_in, vals_a, n, passes);
   } else if (sort_items(n) == kSmallItems) {
     radix_sort_passes<kSmallItems>(keys_a, keys_b, vals_a, vals_b, vals_in, n, work, err, passes, sys_off, nsys, s);
+  } else if (sort_items(n) == kMidItems) {
+    radix_sort_passes<kMidItems>(keys_a, keys_b, vals_a, vals_b, vals_in, n, work, err, passes, sys_off, nsys, s);
   } else {
     radix_sort_passes<kLargeItems>(keys_a, keys_b, vals_a, vals_b, vals_in, n, work, err, passes, sys_off, nsys, s);
   }

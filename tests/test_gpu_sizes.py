@@ -1,6 +1,6 @@
 """Sizes at which a kernel takes another path or a partial tile: the tree's
 1024-position tiles, one narrow level or a grid of them in the multipoles, the
-sort's single block (4096 keys) and its tile sizes (2^19), walk groups shared by
+sort's single block (4096 keys) and its tile sizes (2^17, 2^20), walk groups shared by
 two warps, and the copies of device arrays.  Build results are whole numbers:
 equal to the oracle; forces of shared groups equal, bit for bit, those of the
 same system inside an ensemble too large for sharing."""
@@ -27,7 +27,7 @@ def _tree(pos, nleaf, ncrit, ls=5):
 @pytest.mark.parametrize("n,nleaf,ncrit,same", [
     (1, 16, 64, 0), (2, 1, 1, 0), (33, 16, 64, 0), (1023, 1, 64, 0), (1024, 64, 128, 0), (1025, 16, 64, 0),
     (4095, 8, 32, 0), (4096, 16, 64, 0), (4097, 16, 64, 0), (8193, 63, 16, 0), (5000, 5, 64, 2000),
-    (1 << 19, 16, 64, 0), ((1 << 19) + 1, 16, 64, 0), ((1 << 20) + 3, 16, 64, 0)])
+    (1 << 17, 16, 64, 0), ((1 << 17) + 1, 16, 64, 0), (1 << 20, 16, 64, 0), ((1 << 20) + 3, 16, 64, 0)])
 @pytest.mark.filterwarnings("ignore:.*deeper than 21 levels")
 def test_build_matches_oracle(oracle, lib, n, nleaf, ncrit, same):
     pos, _ = oracle.plummer_float4(n, n % 97 + 1)
