@@ -339,7 +339,9 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&g_count, (size_t)1 << (3 * kMaxLevelSplit)));
     BONSAI_CUDA_TRY(dalloc(&g_seg, (size_t)1 << (3 * kMaxLevelSplit)));
     BONSAI_CUDA_TRY(dalloc(&g_ng, (size_t)1 << (3 * kMaxLevelSplit)));
-    for (int k = 0; k < kWalkVariants; k++) walk_blocks[k] = nsm * walk_blocks_per_sm(k);
+    for (int k = 0; k < 6; k++) walk_blocks[k] = nsm * walk_blocks_per_sm(k);
+    constexpr int shared_of[kWalkVariants - 6] = {0, 1, 3, 4};
+    for (int k = 6; k < kWalkVariants; k++) walk_blocks[k] = walk_blocks[shared_of[k - 6]];
     ring_warps = *std::max_element(walk_blocks, walk_blocks + kWalkVariants) * (kWalkThreads / 32);
     BONSAI_CUDA_TRY(dalloc(&ring, (size_t)ring_warps * kRingCap));
     BONSAI_CUDA_TRY(dalloc(&group_counter, 1));

@@ -749,31 +749,29 @@ static int occupancy(K kernel) {
 
 // blocks per SM that every instantiation of the variant reaches (the level
 // lists are sized for the largest grid)
-template <int NI, bool SPLIT, bool SHARE>
+template <int NI, bool SPLIT>
 static int occupancy_of() {
-  int nb = occupancy(k_walk<NI, SPLIT, false, false, false, SHARE>);
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, false, false, SHARE>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, true, false, SHARE>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, true, false, SHARE>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, true, true, SHARE>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, true, true, SHARE>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, false, true, SHARE>));
-  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, false, true, SHARE>));
+  int nb = occupancy(k_walk<NI, SPLIT, false, false, false, false>);
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, false, false, false>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, true, false, false>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, true, false, false>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, true, true, false>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, true, true, false>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, false, false, true, false>));
+  nb = std::min(nb, occupancy(k_walk<NI, SPLIT, true, false, true, false>));
   return nb < 1 ? 1 : nb;
 }
 
+// (the shared forms take the grid of their unshared ones: no block waits for
+// another, so a grid need not be resident at once)
 int walk_blocks_per_sm(int variant) {
   switch (variant) {
-    case 0: return occupancy_of<1, true, false>();
-    case 1: return occupancy_of<2, true, false>();
-    case 2: return occupancy_of<4, true, false>();
-    case 3: return occupancy_of<1, false, false>();
-    case 4: return occupancy_of<2, false, false>();
-    case 5: return occupancy_of<4, false, false>();
-    case 6: return occupancy_of<1, true, true>();
-    case 7: return occupancy_of<2, true, true>();
-    case 8: return occupancy_of<1, false, true>();
-    default: return occupancy_of<2, false, true>();
+    case 0: return occupancy_of<1, true>();
+    case 1: return occupancy_of<2, true>();
+    case 2: return occupancy_of<4, true>();
+    case 3: return occupancy_of<1, false>();
+    case 4: return occupancy_of<2, false>();
+    default: return occupancy_of<4, false>();
   }
 }
 
