@@ -218,7 +218,7 @@ struct Handle {
     const size_t N = (size_t)n;
     for (int p = 0; p < 2; p++) {
       BONSAI_CUDA_TRY(dalloc(&plo[p], N));
-      BONSAI_CUDA_TRY(cudaMemset(plo[p], 0, N * sizeof(float4)));
+      BONSAI_CUDA_TRY(cudaMemsetAsync(plo[p], 0, N * sizeof(float4), st));
     }
     BONSAI_CUDA_TRY(dalloc(&jlo, N));
     BONSAI_CUDA_TRY(dalloc(&cell_lo, (size_t)cap_cells));
@@ -242,7 +242,7 @@ struct Handle {
     if (bts_K < 0 || n == 0) return 0;
     for (int p = 0; p < 2; p++) {
       BONSAI_CUDA_TRY(dalloc(&lev[p], (size_t)n));
-      BONSAI_CUDA_TRY(cudaMemset(lev[p], 0, (size_t)n));
+      BONSAI_CUDA_TRY(cudaMemsetAsync(lev[p], 0, (size_t)n, st));
     }
     BONSAI_CUDA_TRY(dalloc(&acc_alt, (size_t)n));
     BONSAI_CUDA_TRY(dalloc(&walk_list, (size_t)n));
@@ -313,6 +313,8 @@ struct Handle {
     return 0;
   }
 
+  // (here and in the allocations below: initial contents are set on the
+  // handle's stream, which does not wait for the default stream)
   int init(const bonsai_params* p) {
     prm = *p;
     dev = p->device;
@@ -335,7 +337,7 @@ struct Handle {
     box_blocks = nsm * 4;
     move_blocks = nsm * 4;
     BONSAI_CUDA_TRY(dalloc(&info, 1));
-    BONSAI_CUDA_TRY(cudaMemset(info, 0, sizeof(TreeInfo)));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(TreeInfo), st));
     BONSAI_CUDA_TRY(dalloc(&g_count, (size_t)1 << (3 * kMaxLevelSplit)));
     BONSAI_CUDA_TRY(dalloc(&g_seg, (size_t)1 << (3 * kMaxLevelSplit)));
     BONSAI_CUDA_TRY(dalloc(&g_ng, (size_t)1 << (3 * kMaxLevelSplit)));
@@ -348,25 +350,26 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&stats, 4));
     BONSAI_CUDA_TRY(dalloc(&move_partial, (size_t)move_blocks * 8));
     BONSAI_CUDA_TRY(dalloc(&energies, 8));
-    BONSAI_CUDA_TRY(cudaMemset(energies, 0, 8 * sizeof(double)));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(energies, 0, 8 * sizeof(double), st));
     BONSAI_CUDA_TRY(dalloc(&move_ticket, 1));
     BONSAI_CUDA_TRY(dalloc(&box_ticket, 1));
     BONSAI_CUDA_TRY(dalloc(&mp_barrier, 1));
     BONSAI_CUDA_TRY(dalloc(&f64_odd, 4));
     BONSAI_CUDA_TRY(dalloc(&order_count, 2));
     mp_level_blocks = multipole_level_blocks(nsm);
-    BONSAI_CUDA_TRY(cudaMemset(move_ticket, 0, sizeof(unsigned)));
-    BONSAI_CUDA_TRY(cudaMemset(box_ticket, 0, sizeof(unsigned)));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(move_ticket, 0, sizeof(unsigned), st));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(box_ticket, 0, sizeof(unsigned), st));
     BONSAI_CUDA_TRY(dalloc(&closing, 1));
-    BONSAI_CUDA_TRY(cudaMemset(closing, 0, sizeof(int)));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(closing, 0, sizeof(int), st));
     BONSAI_CUDA_TRY(dalloc(&acc_valid, 2));
-    BONSAI_CUDA_TRY(cudaMemset(acc_valid, 0, 2 * sizeof(int)));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(acc_valid, 0, 2 * sizeof(int), st));
     BONSAI_CUDA_TRY(dalloc(&box, 1));
     BONSAI_CUDA_TRY(dalloc(&box_partial, (size_t)box_blocks * 6));
     std::vector<uint16_t> tab(kPhTableSize);
     build_ph_table(tab.data());
     BONSAI_CUDA_TRY(dalloc(&ph_table, kPhTableSize));
-    BONSAI_CUDA_TRY(cudaMemcpy(ph_table, tab.data(), kPhTableSize * sizeof(uint16_t), cudaMemcpyHostToDevice));
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(ph_table, tab.data(), kPhTableSize * sizeof(uint16_t), cudaMemcpyHostToDevice, st));
+    BONSAI_CUDA_TRY(cudaStreamSynchronize(st));  // the host table goes out of scope
     cur_nleaf = p->nleaf;
     cur_ncrit = p->ncrit;
     cur_ls = p->level_split;
@@ -383,7 +386,7 @@ struct Handle {
       BONSAI_CUDA_TRY(dalloc(&id[p], N));
     }
     BONSAI_CUDA_TRY(dalloc(&acc, N));
-    BONSAI_CUDA_TRY(cudaMemset(acc, 0, N * sizeof(float4)));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(acc, 0, N * sizeof(float4), st));
     BONSAI_CUDA_TRY(dalloc(&jpos, N));
     BONSAI_CUDA_TRY(dalloc(&tkey, N));
     BONSAI_CUDA_TRY(dalloc(&pkey, N));
@@ -400,7 +403,7 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&bsum, (size_t)scan_blocks(scan_m) + 1));
     BONSAI_CUDA_TRY(dalloc(&chain, N));
     BONSAI_CUDA_TRY(dalloc(&hist, tree_hist_words(nn)));
-    BONSAI_CUDA_TRY(cudaMemset(hist, 0, tree_hist_words(nn) * sizeof(unsigned)));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(hist, 0, tree_hist_words(nn) * sizeof(unsigned), st));
     BONSAI_CUDA_TRY(dalloc(&groups, N));
     if (nn <= kOrderMax) BONSAI_CUDA_TRY(dalloc(&group_order, N));
     // group-indexed arrays of the per-group angle: at most N/nCrit groups plus
@@ -410,10 +413,10 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&group_tau, (size_t)gcap));
     BONSAI_CUDA_TRY(dalloc(&group_amag, (size_t)gcap));
     BONSAI_CUDA_TRY(dalloc(&group_stats, (size_t)gcap));
-    BONSAI_CUDA_TRY(cudaMemset(group_stats, 0, (size_t)gcap * sizeof(float4)));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(group_stats, 0, (size_t)gcap * sizeof(float4), st));
     BONSAI_CUDA_TRY(dalloc(&part_gid, N));
-    BONSAI_CUDA_TRY(cudaMemset(part_gid, 0, N * sizeof(int)));
-    BONSAI_CUDA_TRY(cudaMemset(acc_valid, 0, 2 * sizeof(int)));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(part_gid, 0, N * sizeof(int), st));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(acc_valid, 0, 2 * sizeof(int), st));
     BONSAI_CUDA_TRY(dalloc(&group_feat, (size_t)gcap * kMlpFeatures));
     BONSAI_CUDA_TRY(dalloc(&group_counts, (size_t)gcap));
     // the reference reserves nPtcl cells (Treecode.h:192); a Plummer tree at
@@ -463,11 +466,12 @@ struct Handle {
     BONSAI_CUDA_TRY(dalloc(&nseg, 1));
     BONSAI_CUDA_TRY(dalloc(&chunk_energy, (size_t)nchunks * 8));
     BONSAI_CUDA_TRY(dalloc(&sys_energy, (size_t)ns * 8));
-    BONSAI_CUDA_TRY(cudaMemcpy(sys_off, off.data(), (ns + 1) * sizeof(int), cudaMemcpyHostToDevice));
-    BONSAI_CUDA_TRY(cudaMemcpy(chunk_beg, cbeg.data(), (ns + 1) * sizeof(int), cudaMemcpyHostToDevice));
-    BONSAI_CUDA_TRY(cudaMemcpy(chunks, ch.data(), ch.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    BONSAI_CUDA_TRY(cudaMemset(sys_energy, 0, (size_t)ns * 8 * sizeof(double)));
-    BONSAI_CUDA_TRY(cudaMemset(root_beg, 0, (size_t)(ns + 1) * sizeof(int)));
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(sys_off, off.data(), (ns + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(chunk_beg, cbeg.data(), (ns + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(chunks, ch.data(), ch.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+    BONSAI_CUDA_TRY(cudaStreamSynchronize(st));  // the host vectors go out of scope
+    BONSAI_CUDA_TRY(cudaMemsetAsync(sys_energy, 0, (size_t)ns * 8 * sizeof(double), st));
+    BONSAI_CUDA_TRY(cudaMemsetAsync(root_beg, 0, (size_t)(ns + 1) * sizeof(int), st));
     theta_mode = 0;  // angles, precision and block steps are set again for the ensemble
     precision = 0;
     release_lo();
