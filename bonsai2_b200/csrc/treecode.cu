@@ -189,6 +189,7 @@ struct Handle {
   cudaGraphExec_t gexec[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
   int graph_kernels = 0;
   bool graph_ok = false, phases_ok = false;
+  float4* graph_acc = nullptr;  // the acceleration buffer that the graphs write
 
   ~Handle() { release(); }
 
@@ -660,11 +661,20 @@ struct Handle {
     }
     par = par0;
     graph_ok = rc == 0;
+    graph_acc = acc;
     return rc;
+  }
+  // Block steps swap the two acceleration buffers; the graphs hold the one that
+  // was current at their capture.
+  int graph_acc_current() {
+    if (acc == graph_acc) return 0;
+    BONSAI_CUDA_TRY(cudaMemcpyAsync(graph_acc, acc, (size_t)n * sizeof(float4), cudaMemcpyDeviceToDevice, st));
+    std::swap(acc, acc_alt);
+    return 0;
   }
   int capture_phases() {
     const int par0 = par;
-    int rc = 0;
+    int rc = graph_acc_current();
     for (int p = 0; p < 2 && !rc; p++) {
       par = p;
       for (int k = 0; k < 3 && !rc; k++) rc = capture_one(k, &gexec[p][k], nullptr);
@@ -676,6 +686,8 @@ struct Handle {
 
   // ev: four events around the phases, or null for the whole step at once
   int launch_graph_step(cudaEvent_t* ev) {
+    const int rc = graph_acc_current();
+    if (rc) return rc;
     if (!ev) {
       BONSAI_CUDA_TRY(cudaGraphLaunch(gstep[par], st));
     } else {

@@ -1,4 +1,6 @@
 """Block time steps (per-particle power-of-two steps, kick-drift-kick)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -136,3 +138,51 @@ def test_block_steps_in_an_ensemble_are_each_system_alone():
         assert np.array_equal(u.levels(), lev[b:e]), f"levels of system {s}"
         np.testing.assert_allclose(u.computeEnergies(), es[s], rtol=1e-12, atol=1e-15)
         u.close()
+
+
+def _mixed(n, K, graph, calls, theta_mode=0):
+    """The calls on a fresh handle, steps by graph or by plain launches;
+    results after each."""
+    import bonsai2_b200 as B
+    p, v = B.plummer(n, 5)
+    t = B.Treecode(**PRM)
+    _load(t, p, v)
+    t.set_block_steps(K, 0.1)
+    if theta_mode:
+        assert t._L.bonsai_set_theta_mode(t.handle, theta_mode, 1e-2, 1e-2) == 0
+    out = []
+    for c in calls:
+        if c == "step":
+            t.step(1, graph=graph)
+        elif c == "timed":
+            if graph:
+                ms = np.zeros(5, np.float32)
+                assert t._L.bonsai_step_timed(t.handle, 1, ms.ctypes.data_as(ctypes.c_void_p)) == 0
+            else:
+                t.step(1, graph=False)
+        elif c == "block":
+            t.block_step(1)
+        elif c == "load":
+            t.ptcl_h2d()
+        assert t.synchronize() == 0
+        t.ptcl_d2h()
+        out.append((t.h_ptclPos.copy(), t.h_ptclVel.copy(), t.get_acc(), None if c == "load" else t.computeEnergies()))
+    t.close()
+    return out
+
+
+@pytest.mark.parametrize("theta_mode", [0, 3])
+@pytest.mark.parametrize("K", [0, 2])
+@pytest.mark.parametrize("calls", [
+    # the second block step of level 0 swaps the acceleration buffers an odd number of times
+    ("step", "block", "block", "step", "load", "step"),
+    ("step", "block", "block", "timed", "step", "timed"),
+])
+def test_graph_steps_between_block_steps(theta_mode, K, calls):
+    """Steps replayed from graphs after block steps give what plainly launched
+    ones give: the graphs hold the buffers of the capture."""
+    a, b = (_mixed(8000, K, graph, calls, theta_mode) for graph in (True, False))
+    for k, (x, y) in enumerate(zip(a, b)):
+        for q, (u, w) in enumerate(zip(x, y)):
+            assert (u is None) == (w is None)
+            assert u is None or np.array_equal(u, w), (k, calls[k], q)
