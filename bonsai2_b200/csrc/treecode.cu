@@ -650,16 +650,28 @@ struct Handle {
     cudaGraphDestroy(g);
     return e == cudaSuccess ? 0 : -(int)e - 1000;
   }
+  // What enqueuing a step notes about the state's order.  A capture runs nothing,
+  // so it leaves all of it as it was; a replay notes it in launch_graph_step.
+  struct StateOrder {
+    int par;
+    bool bts_ready, acc_in_state_order;
+  };
+  StateOrder state_order() const { return {par, bts_ready, acc_in_state_order}; }
+  void set_state_order(const StateOrder& o) {
+    par = o.par;
+    bts_ready = o.bts_ready;
+    acc_in_state_order = o.acc_in_state_order;
+  }
   int capture_graphs() {
     release_graphs();
-    const int par0 = par;
+    const StateOrder before = state_order();
     graph_kernels = 0;
     int rc = 0;
     for (int p = 0; p < 2 && !rc; p++) {
       par = p;
       rc = capture_one(-1, &gstep[p], p == 0 ? &graph_kernels : nullptr);
     }
-    par = par0;
+    set_state_order(before);
     graph_ok = rc == 0;
     graph_acc = acc;
     return rc;
@@ -673,13 +685,13 @@ struct Handle {
     return 0;
   }
   int capture_phases() {
-    const int par0 = par;
+    const StateOrder before = state_order();
     int rc = graph_acc_current();
     for (int p = 0; p < 2 && !rc; p++) {
       par = p;
       for (int k = 0; k < 3 && !rc; k++) rc = capture_one(k, &gexec[p][k], nullptr);
     }
-    par = par0;
+    set_state_order(before);
     phases_ok = rc == 0;
     return rc;
   }
@@ -697,7 +709,7 @@ struct Handle {
       }
       BONSAI_CUDA_TRY(cudaEventRecord(ev[3], st));
     }
-    par ^= 1;
+    set_state_order({par ^ 1, false, true});
     return 0;
   }
 

@@ -162,6 +162,9 @@ def _mixed(n, K, graph, calls, theta_mode=0):
                 t.step(1, graph=False)
         elif c == "block":
             t.block_step(1)
+        elif c == "capture":
+            if graph:
+                assert t._L.bonsai_graph_kernel_count(t.handle) > 0
         elif c == "load":
             t.ptcl_h2d()
         assert t.synchronize() == 0
@@ -176,11 +179,14 @@ def _mixed(n, K, graph, calls, theta_mode=0):
 @pytest.mark.parametrize("calls", [
     # the second block step of level 0 swaps the acceleration buffers an odd number of times
     ("step", "block", "block", "step", "load", "step"),
-    ("step", "block", "block", "timed", "step", "timed"),
+    ("block", "step", "block", "step", "block", "step", "step"),
+    ("step", "block", "block", "timed", "step", "timed", "block", "timed"),
+    ("block", "capture", "block", "capture", "block"),
 ])
 def test_graph_steps_between_block_steps(theta_mode, K, calls):
-    """Steps replayed from graphs after block steps give what plainly launched
-    ones give: the graphs hold the buffers of the capture."""
+    """Steps replayed from graphs between block steps give what plainly
+    launched ones give: the graphs hold the addresses of the capture, and a
+    replay runs none of the host's bookkeeping."""
     a, b = (_mixed(8000, K, graph, calls, theta_mode) for graph in (True, False))
     for k, (x, y) in enumerate(zip(a, b)):
         for q, (u, w) in enumerate(zip(x, y)):
