@@ -153,7 +153,7 @@ void launch_closing_kick(float4* vel, const float4* acc, int n, float dt, int* c
 // FP64 direct sum inside each sample's own system (one block per sample; lo as launch_direct_fp64)
 void launch_direct_fp64_sys(const float4* pos, const int* sys_off, int nsys, const int* sample, int ns, double eps2,
                             int include_self, double* out, cudaStream_t s, const float4* lo = nullptr);
-// slices of the sources (nsplit) that fill the device once
+// slices of the sources (nsplit) for ns samples
 int direct_slices(int ns, int nsm);
 // lo (nullable): double-single low parts, positions taken as hi + lo
 void launch_direct_fp64(const float4* pos, int n, const int* sample, int ns, double eps2, int include_self,

@@ -194,12 +194,17 @@ void launch_move(float4* pos, float4* vel, const float4* acc, int n, float dt, i
 // nsplit); thread = one sample, block = one slice of the sources.  A sample
 // index outside [0, n) reads nothing: its partial sums are NaN, so its output
 // row is NaN (the allocation-free entry point passes caller device indices
-// that no host code has checked).
+// that no host code has checked).  A slice is summed tile by tile, each tile's
+// 256 terms by themselves: one running sum per slice grew its error with the
+// slice.  4096 samples of 2^18 particles against 80-bit sums, relative error:
+// 1.0e-16 with the runs of the fold below (Plummer; clustered field 1.6e-16),
+// 3.2e-16 (4.8e-16) with running sums over 74 slices, 3.6e-16 (9.2e-16) over 46.
 __global__ void __launch_bounds__(256) k_direct_fp64(const float4* __restrict__ pos, int n,
                                                      const int* __restrict__ sample, int ns, double eps2,
                                                      int include_self, double* __restrict__ part,
                                                      const float4* __restrict__ lo) {
   __shared__ double4 sj[256];
+  __shared__ double tot[4][256];  // in registers they would cost a block per SM
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int nsplit = gridDim.y;
   const int jb = (int)((long long)n * blockIdx.y / nsplit), je = (int)((long long)n * (blockIdx.y + 1) / nsplit);
@@ -212,7 +217,8 @@ __global__ void __launch_bounds__(256) k_direct_fp64(const float4* __restrict__ 
     const float4 l = lo[i];
     xi += l.x; yi += l.y; zi += l.z;
   }
-  double ax = 0, ay = 0, az = 0, ph = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) tot[k][threadIdx.x] = 0.0;
   for (int j0 = jb; j0 < je; j0 += 256) {
     __syncthreads();
     const int jj = j0 + threadIdx.x;
@@ -227,6 +233,7 @@ __global__ void __launch_bounds__(256) k_direct_fp64(const float4* __restrict__ 
     }
     __syncthreads();
     const int cnt = min(256, je - j0);
+    double ax = 0, ay = 0, az = 0, ph = 0;
     auto add = [&](int t) {
       const double4 q = sj[t];
       const double dx = q.x - xi, dy = q.y - yi, dz = q.z - zi;
@@ -245,38 +252,57 @@ __global__ void __launch_bounds__(256) k_direct_fp64(const float4* __restrict__ 
 #pragma unroll 4
       for (int t = 0; t < cnt; t++) add(t);
     }
+    tot[0][threadIdx.x] += ax; tot[1][threadIdx.x] += ay; tot[2][threadIdx.x] += az; tot[3][threadIdx.x] += ph;
   }
   if (s < ns) {
-    if (!valid) ax = ay = az = ph = __longlong_as_double(0x7ff8000000000000LL);
     double* o = part + ((size_t)blockIdx.y * ns + s) * 4;
-    o[0] = ax; o[1] = ay; o[2] = az; o[3] = ph;
+#pragma unroll
+    for (int k = 0; k < 4; k++) o[k] = valid ? tot[k][threadIdx.x] : __longlong_as_double(0x7ff8000000000000LL);
   }
 }
 
-__global__ void k_direct_fold(const double* __restrict__ part, int ns, int nsplit, double* __restrict__ out) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * ns; t += gridDim.x * blockDim.x) {
-    double x = 0;
+// The slices' sums added in eight runs of slices, then the runs: one sum over
+// all slices has more error than the slices themselves (512 of them, 6.3e-16
+// against 1.2e-16 in runs), and a thread for it is slow (1000 samples of 4096
+// particles in 185 slices 64 us, 51 with a warp for each run).
+__global__ void __launch_bounds__(256) k_direct_fold(const double* __restrict__ part, int ns, int nsplit,
+                                                     double* __restrict__ out) {
+  __shared__ double sh[8][32];
+  const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
+  const size_t t = (size_t)blockIdx.x * 32 + lane, m = (size_t)ns * 4;
+  double x = 0;
+  if (t < m) {
+    const int e = nsplit * (run + 1) / 8;
 #pragma unroll 8
-    for (int q = 0; q < nsplit; q++) x += part[(size_t)q * ns * 4 + t];
-    out[t] = x;
+    for (int q = nsplit * run / 8; q < e; q++) x += part[q * m + t];
   }
+  sh[run][lane] = x;
+  __syncthreads();
+  if (run || t >= m) return;
+  double y = 0;
+#pragma unroll
+  for (int q = 0; q < 8; q++) y += sh[q][lane];
+  out[t] = y;
 }
 
-// Slices of the sources for ns samples: as many blocks as are resident at once,
-// so that all of them run in one wave.  (1184 blocks of 4096 samples on 740 places
-// took two: 2^18 sources 1.63 -> 1.45 ms, 73 % of the FP64 pipe at 18 operations
-// an interaction.)
+// Slices of the sources for ns samples.  Every block of 256 samples and a slice
+// takes the same time and the FP64 pipe is the bound however many of an SM's
+// blocks are resident, so the blocks are a whole number per SM, up to 20 of
+// them: the fewer, the longer an SM waits for the last block at the end (n =
+// 250,007, slices and ms: 1000 samples 185 0.387, 481 0.373; 4096 samples 46
+// 1.430, 92 1.369, 185 1.332; 65,536 samples 2 26.3, 4 21.6, 12 20.7; 189,000
+// samples 1 63.1, 4 58.9).  At most 512 slices (the scratch).
 int direct_slices(int ns, int nsm) {
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_direct_fp64, 256, 0) != cudaSuccess || occ < 1) occ = 1;
-  return std::max(1, std::min(512, nsm * occ / ((ns + 255) / 256)));
+  const long long blocks = (ns + 255ll) / 256;
+  const long long per_sm = std::min(20ll, 512 * blocks / nsm);
+  return (int)std::max(1ll, std::min(512ll, per_sm * nsm / blocks));
 }
 
 void launch_direct_fp64(const float4* pos, int n, const int* sample, int ns, double eps2, int include_self,
                         double* part, int nsplit, double* out, cudaStream_t s, const float4* lo) {
   dim3 grid((ns + 255) / 256, nsplit);
   k_direct_fp64<<<grid, 256, 0, s>>>(pos, n, sample, ns, eps2, include_self, part, lo);
-  k_direct_fold<<<(4 * ns + 255) / 256, 256, 0, s>>>(part, ns, nsplit, out);
+  k_direct_fold<<<(unsigned)((4ll * ns + 31) / 32), 256, 0, s>>>(part, ns, nsplit, out);
 }
 
 // The pending closing kick v += a dt/2 (the same operation the move applies

@@ -154,3 +154,31 @@ def test_autotune_restores_double_single_state():
     assert np.array_equal(before[0].view(np.uint64), after[0].view(np.uint64))
     assert np.array_equal(before[1].view(np.uint32), after[1].view(np.uint32))
     t.close()
+
+
+@pytest.mark.parametrize("eps", [0.7, 1.1, 1.7, 2.3, 3.1])
+@pytest.mark.parametrize("ns", [1, 4096])
+def test_direct_sum_rounding(lib, eps, ns):
+    """FP64 direct sum of 2^18 equal terms (particles at one point) against
+    2^18 times the one term, which is exact.  A sum of k terms is off by at most
+    k - 1 roundings of 2^-53: 255 in a tile, the tiles of a slice, the slices of a
+    run and the eight runs (4096 samples: 185 slices of 6 tiles, runs of 24; one
+    sample: 444 of 3, runs of 56; 148 SMs)."""
+    import bonsai2_b200 as B
+    n = 1 << 18
+
+    def potential(count):
+        pos = np.zeros((count, 4), np.float32)
+        pos[:, 3] = 0.3
+        t = B.Treecode(eps=eps)
+        t.alloc(count)
+        t.h_ptclPos[:] = pos
+        t.ptcl_h2d()
+        d = t.direct_fp64(np.arange(min(ns, count), dtype=np.int32))
+        t.close()
+        assert not d[:, :3].any()
+        return d[:, 3]
+
+    one = potential(1)[0]
+    bound = (255 + 5 + 23 + 7 if ns == 4096 else 255 + 2 + 55 + 7) * 2.0 ** -53
+    assert np.abs(potential(n) / (n * one) - 1).max() <= bound
