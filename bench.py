@@ -1,6 +1,10 @@
 #!/usr/bin/env python
 """Full-step throughput of the B200 tree code (one JSON line on rank 0).
 
+The line is the result with the main figures of each form; the whole record
+(sweeps, learned form, ensembles, precision, block steps, with their parameters)
+goes to stderr as one JSON line, and to --report FILE.
+
 Workload (the large Plummer configuration): N = 2^24 equal-mass Plummer
 sphere (seeded, the reference's plummer.h algorithm), float32, eps = 0.005,
 NLEAF = 16, NCRIT = 64, levelSplit = 5, dt = 1/128, fixed-theta FP32 walk.
@@ -100,6 +104,7 @@ def parse():
     ap.add_argument("--e2e-steps", type=int, default=20,
                     help="pipelined end-to-end steps (the first upload and the last download are not overlapped)")
     ap.add_argument("--error-samples", type=int, default=4096)
+    ap.add_argument("--report", default="", help="also write the whole record (JSON) to this file")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--cpu-group-fraction", type=float, default=1.0 / 512)
     return ap.parse_args()
@@ -366,6 +371,43 @@ def bench_config(a, world):
             "l2": "no flush: particle state 1.3 GB > 126 MB L2"}
 
 
+# what the result line keeps of the whole record: these keys as they are, of each
+# form its main figures, of the sweep a row per theta.  A line of all of it is over
+# 20 KB, more than readers of a log's tail get.
+LINE_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+             "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "clocks", "roofline", "cpu_baseline",
+             "accuracy", "stages_ms", "status")
+FORM_KEYS = ("value", "ms_per_step", "ms_per_big_step", "ms", "theta", "median_rel_force_err", "gain_at_equal_median",
+             "vs_best_fixed_meeting_target", "vs_published", "ds_cost", "frac", "unavailable")
+MAX_LINE = 4000
+
+
+def result_line(record):
+    """The result line (a string of at most MAX_LINE characters) of a whole record."""
+    def short(x):
+        if isinstance(x, float):
+            return float("%.7g" % x)
+        if isinstance(x, dict):
+            return {k: short(v) for k, v in x.items()}
+        return [short(v) for v in x] if isinstance(x, (list, tuple)) else x
+
+    line = {k: record[k] if k in ("value", "ms_per_step") else short(record[k]) for k in LINE_KEYS if k in record}
+    forms = {}
+    for name, form in record.items():
+        if name in LINE_KEYS or not isinstance(form, dict):
+            continue
+        kept = {k: short(form[k]) for k in FORM_KEYS if isinstance(form.get(k), (int, float, str))}
+        if kept:
+            forms[name] = kept
+    if record.get("theta_sweep"):
+        forms["theta_sweep"] = [short([r["theta"], r["value"], r["median_rel_force_err"]]) for r in record["theta_sweep"]]
+    for part in ({"forms": forms}, {}):
+        text = json.dumps(dict(line, **part))
+        if len(text) <= MAX_LINE:
+            break
+    return text
+
+
 def run_reference(a):
     d = Dist("gloo")
     if d.rank != 0:
@@ -596,7 +638,12 @@ def run_ours(a):
         if learned:
             learned["vs_fixed_headline"] = learned["value"] / value
             learned["double_single"]["vs_fixed_headline"] = learned["double_single"]["value"] / value
-        print(json.dumps(line), flush=True)
+        whole = json.dumps(line)
+        if a.report:
+            with open(a.report, "w") as f:
+                f.write(whole + "\n")
+        print(whole, file=sys.stderr, flush=True)
+        print(result_line(line), flush=True)
     for hptr in (hp, hv, ha):
         L.bonsai_host_free(hptr)
     d.close()

@@ -44,3 +44,33 @@ def test_workload_names_the_configuration():
                               seed=19810614)
     w = bench.workload(a)
     assert "N=16777216" in w and "theta=0.6" in w and "dt=1/128" in w and "FP32" in w
+
+
+def test_result_line_is_short_and_whole():
+    """The line that rank 0 prints carries every figure of the result and stays
+    within what a log's tail holds, however long the record."""
+    import json
+    import bench
+    row = {"theta": 0.6, "value": 1.0 / 3, "median_rel_force_err": 2.6e-4 / 3, "what": "x" * 500}
+    form = {"value": 1.0 / 3, "ms_per_step": 2.0 / 3, "sweep": [row] * 20, "what": "y" * 2000}
+    record = {"metric": bench.METRIC, "value": 245.123456789, "unit": bench.UNIT, "n_gpus": 1, "steps": 20, "warmup": 5,
+              "ms_per_step": 68.123456789, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
+              "dtype": "f32", "data": "synthetic", "gpu_launches": 760,
+              "config": {"workload": "w" * 120, "n_per_gpu": 1 << 24, "parallelism": "replicas x1", "l2": "no flush"},
+              "e2e": {"value": 1.0 / 3, "unit": bench.UNIT, "h2d_bytes_per_step": 1 << 29, "d2h_bytes_per_step": 1 << 28},
+              "clocks": {"sm_mhz": 1965.0, "sm_max_mhz": 1965.0, "reasons": []},
+              "roofline": {"bound": "fp32", "frac": 1.0 / 3}, "theta_sweep": [row] * 8, "skipped_form": None,
+              **{"form%d" % k: dict(form) for k in range(9)}}
+    line = bench.result_line(record)
+    assert "\n" not in line and len(line) <= bench.MAX_LINE
+    got = json.loads(line)
+    for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+              "vs_baseline", "dtype", "data", "gpu_launches", "config", "clocks"):
+        assert got[k] == record[k], k
+    assert got["e2e"]["value"] == pytest.approx(1.0 / 3, rel=1e-6) and got["e2e"]["h2d_bytes_per_step"] == 1 << 29
+    assert got["forms"]["form3"]["value"] == pytest.approx(1.0 / 3, rel=1e-6)
+    assert len(got["forms"]["theta_sweep"]) == 8
+    # forms that do not fit are left out, the result never
+    record.update({"f%d" % k: dict(form) for k in range(200)})
+    line = bench.result_line(record)
+    assert len(line) <= bench.MAX_LINE and json.loads(line)["value"] == record["value"]
