@@ -55,6 +55,7 @@ void build_tree(const unsigned long long* sorted_keys, int n, int nleaf, int cel
 // double-single positions)
 // barrier: one word of scratch; level_blocks: multipole_level_blocks of the device
 int multipole_level_blocks(int nsm);
+int barrier_timeout_selftest(cudaStream_t s);
 void launch_multipoles(const int* leaf_list, TreeInfo* info, const uint4* cell_data, const float4* jpos, int n,
                        float inv_theta, MpRec* rec, void* box, float4* cell_open, float4* cell_stage,
                        float4* cell_ls, int cell_cap, const float4* jlo, float4* cell_lo, int nblocks,

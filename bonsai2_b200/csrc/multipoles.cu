@@ -151,7 +151,8 @@ constexpr int kBarrierSpin = 1 << 22;  // a few seconds
 
 // All blocks have arrived `round` times.  The wait is bounded: past the bound
 // it reports, and the caller returns (results invalid).
-__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned round, int* status) {
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned round, int* status,
+                                             int limit = kBarrierSpin) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -160,7 +161,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned round, in
     const unsigned target = round * gridDim.x;
     volatile unsigned* c = count;
     int spin = 0;
-    while (*c < target && spin < kBarrierSpin) {
+    while (*c < target && spin < limit) {
       __nanosleep(20);
       spin++;
     }
@@ -503,6 +504,40 @@ void launch_multipoles(const int* leaf_list, TreeInfo* info, const uint4* cell_d
     launch_multipoles_of<false>(leaf_list, info, cell_data, jpos, n, inv_theta, rec, static_cast<float*>(box),
                                 cell_open, cell_stage, cell_ls, cell_cap, nullptr, nullptr, nblocks, barrier,
                                 level_blocks, s);
+}
+
+// Self-test of the level barrier's bound.  Two blocks meet at round 1, and then
+// at round 3 with nobody at round 2: the wait runs out, and both must report and leave.
+__global__ void k_barrier_selftest(unsigned* count, int* status, unsigned* left) {
+  if (!grid_barrier(count, 1, status)) return;
+  const bool late = !grid_barrier(count, 3, status, 1 << 12);
+  if (threadIdx.x == 0 && late) atomicAdd(left, 1u);
+}
+
+// Returns the status bits, 0 when a block did not report (or a CUDA error as -1000 - code).
+int barrier_timeout_selftest(cudaStream_t s) {
+  constexpr unsigned kBlocks = 2;
+  unsigned* word = nullptr;  // arrivals, status, blocks that gave up
+  unsigned host[3] = {0, 0, 0};
+  cudaError_t e = cudaMalloc(&word, sizeof(host));
+  if (e == cudaSuccess) e = cudaMemsetAsync(word, 0, sizeof(host), s);
+  if (e == cudaSuccess) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kBlocks);
+    cfg.blockDim = dim3(64);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, k_barrier_selftest, word, reinterpret_cast<int*>(word + 1), word + 2);
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(host, word, sizeof(host), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaFree(word);
+  if (e != cudaSuccess) return -(int)e - 1000;
+  return host[2] == kBlocks ? (int)host[1] : 0;
 }
 
 // Reference-layout view of the multipoles (debug/parity getter):

@@ -1974,8 +1974,9 @@ int bonsai_selftest_wait_bound(int device) {
   cudaStream_t st;
   BONSAI_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   const int r = sort_timeout_selftest(st);
+  const int b = r < 0 ? 0 : barrier_timeout_selftest(st);
   cudaStreamDestroy(st);
-  return r;
+  return r < 0 ? r : (b < 0 ? b : r & b);
 }
 
 int bonsai_fp32_peak(int device, double* tflops) {

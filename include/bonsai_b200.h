@@ -140,9 +140,11 @@ int bonsai_graph_kernel_count(bonsai_handle h);
 int bonsai_get_stats(bonsai_handle h, unsigned long long *out4);
 /* Failure-detection self-test (no counterpart in the reference, whose waits
  * are unbounded): runs one radix-sort pass whose first tile never starts, so
- * the next tile's look-back waits on a flag nothing sets; the wait must end at
- * its bound and report.  Returns the status bits (BONSAI_STATUS_SORT_TIMEOUT
- * expected) after a fraction of a second; the device stays usable. */
+ * the next tile's look-back waits on a flag nothing sets, and the multipoles'
+ * level barrier for a round that nobody else joins; each wait must end at its
+ * bound and report.  Returns the status bits that both reported
+ * (BONSAI_STATUS_SORT_TIMEOUT expected) after a few seconds; the device stays
+ * usable. */
 int bonsai_selftest_wait_bound(int device);
 /* Bounds-checked builds (the library compiled with -DBONSAI_CHECKS, e.g.
  * `python -m bonsai2_b200.build --checks`): every guarded index of the kernels

@@ -257,7 +257,8 @@ def test_max_size_2p27_invariants():
 def test_bounded_wait_reports_and_device_stays_usable():
     """A radix-sort pass whose first tile never starts: the next tile's
     look-back waits on a flag nothing sets, ends at its bound and reports
-    BONSAI_STATUS_SORT_TIMEOUT; the device then runs a normal step."""
+    BONSAI_STATUS_SORT_TIMEOUT; so do all blocks at a round of the multipoles'
+    level barrier that nobody else joins; the device then runs a normal step."""
     import bonsai2_b200 as B
     L = B.load()
     r = L.bonsai_selftest_wait_bound(0)
