@@ -54,23 +54,39 @@ def test_build_matches_oracle(oracle, lib, n, nleaf, ncrit, same):
     t.close()
 
 
-@pytest.mark.parametrize("ncrit,sizes", [(64, (1, 15, 1000, 30011, 85000)), (32, (2, 300, 12001, 14001)),
-                                         (128, (5, 4000, 200001, 330000)), (16, (700, 20000))])
+# each system small enough for shared groups, their ensemble too large (layout 1
+# shares one row of 32 between two warps); groups of nCrit 16 are one row of 16
+# and never shared, alone or together
+@pytest.mark.parametrize("ncrit,layout,sizes", [
+    (64, 0, (1, 15, 1000, 30011, 85000)), (32, 0, (2, 300, 12001, 14001)), (128, 0, (5, 4000, 200001, 330000)),
+    (64, 1, (1, 33, 700, 20011, 40000)), (16, 0, (700, 20000))])
 @pytest.mark.parametrize("precision", [0, 1])
-def test_shared_groups_bit_identical(lib, ncrit, sizes, precision):
+@pytest.mark.parametrize("theta_mode", [0, 1, 3])
+def test_shared_groups_bit_identical(lib, ncrit, layout, sizes, precision, theta_mode):
+    """Four steps: in the network's and the relative mode (1, 3) the first walk is
+    at the fixed angle, and from the third on the features are those of a
+    relative walk's statistics, which one of a shared group's warps records."""
     import bonsai2_b200 as B
+    from bonsai2_b200 import learned
     from bonsai2_b200.ensemble import plummer_ensemble
     counts = np.array(sizes, np.int32)
     pos, vel = plummer_ensemble(counts, base_seed=11)
     prm = dict(eps=0.01, theta=0.7, ncrit=ncrit)
+    w = learned.init_weights(3)
 
     def run(t, p, v):
         if precision:
             t.set_precision(1)
+        t.set_walk_layout(layout)
+        if theta_mode == 1:
+            assert lib.bonsai_set_mlp_weights(t.handle, w.ctypes.data_as(ctypes.c_void_p), w.size) == 0
+        if theta_mode:
+            assert lib.bonsai_set_theta_mode(t.handle, theta_mode, *((1e-2, 1e-2) if theta_mode == 3 else
+                                                                     (learned.YLO, learned.YHI))) == 0
         t.h_ptclPos[:] = p
         t.h_ptclVel[:] = v
         t.ptcl_h2d()
-        t.step(2)
+        t.step(4)
         assert t.synchronize() == 0
         t.ptcl_d2h()
         out = t.h_ptclPos.copy(), t.h_ptclVel.copy(), t.get_acc()

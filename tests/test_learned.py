@@ -59,9 +59,11 @@ def test_gpu_gradient_matches_oracle(lib):
 @pytest.mark.parametrize("S", [1, 63, 64, 65, 148 * 64, 148 * 64 + 1, 30011])
 def test_gpu_gradient_sample_tiles(lib, S):
     """Sizes around the 64-sample tiles and around one tile per block (148
-    blocks).  FP32 sums of at most S / 32 terms per thread: relative error
-    below S / 32 * 2^-24 of the sum of magnitudes, far under the bounds of the
-    test above."""
+    blocks).  Roundings of 2^-24 behind a gradient, as parts of the sum of
+    magnitudes: under 200 in a sample's own chain (products of 16 and 64 terms
+    forward and back, tanhf, expf), 32 per tile of the block (4 tiles at most
+    here), 1 for the block's halves and 27 for the blocks; 2.1e-5 at the very
+    most, against the bounds of the test above."""
     from oracle import mlp_oracle as M
     from bonsai2_b200 import learned as Lr
     X, y = _data(S, seed=S)
