@@ -24,7 +24,8 @@ constexpr int kScanChunk = 4096;
 // tile's latency, 16 where the digit runs that a tile writes out have to be long,
 // 8 between.  Build of a whole step with 4 / 8 / 16 (us): 30,011 particles 126 /
 // 139, 131,072 169 / 171 / 200, 250,007 220 / 212 / 229, 500,000 300 / 297 / 308,
-// 2^20 - / 413 / 450, 1.7M - / 591 / 571.  Same order with any.
+// 2^20 - / 411 / 438, 1.15M - / 452 / 475, 1.5M - / 536 / 544, 1.7M - / 602 / 580:
+// the upper line is short of where the sides meet.  Same order with any.
 constexpr int kSmallItems = 4, kMidItems = 8, kLargeItems = 16;
 constexpr int kSortSmallMax = 1 << 17, kSortMidMax = 1 << 20;
 static int sort_items(int n) { return n <= kSortSmallMax ? kSmallItems : (n <= kSortMidMax ? kMidItems : kLargeItems); }

@@ -1,4 +1,4 @@
-// tree.cu -- octree from the sorted octant-path keys, in three launches and no
+// tree.cu -- octree from the sorted octant-path keys, in four launches and no
 // host round trip.
 //
 // The reference builds the tree by a recursive CUDA-dynamic-parallelism

@@ -727,9 +727,15 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
 //   split, nCrit 32 (NI 2): 16,384 184/133, 40,000 field 160/178
 //   full, nCrit 128 (NI 4): 65,536 971/428, 250,007 galaxy 1463/1102, 500,000
 //     1778/1776 (galaxy 2223/1983), 2^20 3494/3650
-// and as many for the full-warp NI 2, by the particles of its rows, as for the
-// split one.  (Four warps per group were no better than two up to 16,384 and
-// worse above.)
+//   full, nCrit 64 (NI 2): 32,768 431/245, 49,152 455/316 (field 352/298),
+//     65,536 481/369 (field 375/315)
+// The two NI 2 lines are on the safe side: the split form still gains at 32,768
+// (225/193, field 177/147).  The per-group-angle, double-single and ensemble
+// forms were timed at both sides of every line (three distributions): shared
+// over whole 0.43 to 0.97 below it, but for nCrit 128 from 262,144 particles on
+// (0.66 to 1.04).  The line goes by the particles, also where block steps walk
+// part of the groups.  (Four warps per group were no better than
+// two up to 16,384 and worse above.)
 int walk_variant(int n, int ncrit, int layout, int* parts) {
   const bool split = BONSAI_WALK_SPLIT && ncrit <= 64 && layout != 1;
   const int rows = (ncrit + (split ? 15 : 31)) / (split ? 16 : 32);
