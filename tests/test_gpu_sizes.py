@@ -163,6 +163,27 @@ def test_double_positions_round_trip(lib, n, precision):
     t.close()
 
 
+@pytest.mark.parametrize("n,ns", [(1, 1), (7, 3), (300, 1), (300, 257), (2049, 1000), (5000, 5000), (1000, 40000),
+                                  (2000, 200000)])
+@pytest.mark.parametrize("include_self", [True, False])
+def test_direct_sum_slices(oracle, lib, n, ns, include_self):
+    """The direct sum at 444 slices (also of fewer sources), 481, 148, 18 (runs of
+    two and three) and 3 (empty runs).  FP64 on both sides: the difference is
+    a few roundings of 2^-53 for each of at most 5000 terms, 1e-12 of the terms'
+    magnitudes, which the near pairs dominate."""
+    import bonsai2_b200 as B
+    pos, _ = B.plummer(n, 6)
+    t = B.Treecode(eps=0.05)
+    t.alloc(n)
+    t.h_ptclPos[:] = pos
+    t.ptcl_h2d()
+    sample = np.random.default_rng(n).integers(0, n, ns).astype(np.int32)
+    got = t.direct_fp64(sample, include_self)
+    t.close()
+    want = oracle.direct_fp64(pos, sample, 0.05, include_self)
+    assert np.allclose(got, want, rtol=1e-12, atol=1e-12 * max(1.0, np.abs(want).max()))
+
+
 def test_handles_in_threads(lib):
     """Handles stepped from threads of their own at once give what each gives
     alone: their steps share the GPU, grid-wide barriers of the multipoles'
